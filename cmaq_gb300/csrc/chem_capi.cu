@@ -100,6 +100,7 @@ struct cmaqchem_handle {
     int rconst_pass = 1;
     double* d_rki_all = nullptr;
     uint8_t* d_sun_all = nullptr;
+    int coop = -1;           // cooperative ROS3 kernel: -1 by size (use_coop), 0 off, 1 always
     int q_sync = 1;          // work-queue kernel: barriers between attempt phases
     int q_wpb = 8;           // work-queue kernel: warps per block
     int q_nblocks = 0;
@@ -212,6 +213,13 @@ int configure_queue(cmaqchem_handle* h)
     if (h->q_bps_cap > 0 && bps > h->q_bps_cap) bps = h->q_bps_cap;
     h->q_nblocks = h->nsm * bps;
     return ensure_ws(h, (size_t)h->q_nblocks * h->q_wpb);
+}
+
+// Whether a ROS3 call of n cells takes the cooperative kernel (same results): below the
+// mechanism's limit it is faster, above it the one-cell-per-lane kernels fill the device.
+bool use_coop(const cmaqchem_handle* h, long long n)
+{
+    return h->coop >= 0 ? h->coop > 0 : n <= h->ops->coop_limit;
 }
 
 int upload_gear_coef(cmaqchem_handle* h)
@@ -395,7 +403,8 @@ extern "C" int cmaqchem_init(const cmaqchem_cfg* cfg, cmaqchem_handle** out)
         CK(cudaMalloc(&h->d_hist, sizeof(unsigned int) * chem::QUEUE_BINS));
         CK(cudaMalloc(&h->d_cursor, sizeof(unsigned long long) * chem::QUEUE_BINS));
         CK(cudaMalloc(&h->d_head, sizeof(unsigned long long)));
-        if (cfg->solver == CMAQCHEM_SOLVER_ROS3 && cfg->schedule == CMAQCHEM_SCHED_QUEUE) {
+        if (cfg->solver == CMAQCHEM_SOLVER_ROS3 &&
+            (cfg->schedule == CMAQCHEM_SCHED_QUEUE || use_coop(h, h->ncell))) {
             // the rate-constant pass's arrays, when they leave a quarter of the free memory
             const size_t bytes = sizeof(double) * (size_t)m->nrxns * h->ncell;
             size_t free_b = 0, total_b = 0;
@@ -470,6 +479,12 @@ extern "C" int cmaqchem_diag_set_tuning(cmaqchem_handle* h, const char* key, int
         if (h->graph_exec) CK(cudaGraphExecDestroy(h->graph_exec));
         h->graph_exec = nullptr;
         return 0;
+    } else if (strcmp(key, "ros3_coop") == 0) {
+        if (value < -1 || value > 1) return fail("ros3_coop must be -1 (by size), 0 or 1");
+        h->coop = value;
+        if (h->graph_exec) CK(cudaGraphExecDestroy(h->graph_exec));
+        h->graph_exec = nullptr;
+        return 0;
     } else if (strcmp(key, "rconst_pass") == 0) {
         // 1: the work-queue ROS3 call evaluates CALC_RCONST in a pass of whole warps first
         // (when its arrays were allocated at set-up); 0: in the refilled lanes; same numbers
@@ -522,7 +537,8 @@ static int enqueue_step(cmaqchem_handle* h, const chem::GridArgs& a, int itmstep
     const bool gear_solver = h->cfg.solver == CMAQCHEM_SOLVER_GEAR;
     if (c1 < 0) c1 = h->ncell;
     const long long n = c1 - c0;
-    if (h->cfg.schedule == CMAQCHEM_SCHED_QUEUE || ebi_solver || gear_solver) {
+    const bool coop = !ebi_solver && !gear_solver && h->rconst_pass && h->d_rki_all && use_coop(h, n);
+    if (h->cfg.schedule == CMAQCHEM_SCHED_QUEUE || ebi_solver || gear_solver || coop) {
         chem::QueueArgs q{nullptr, h->d_head, n, c0};
         if (sort && (h->cfg.schedule == CMAQCHEM_SCHED_QUEUE || gear_solver)) {
             const int nb = 4 * h->nsm;
@@ -569,7 +585,14 @@ static int enqueue_step(cmaqchem_handle* h, const chem::GridArgs& a, int itmstep
             chem::GridArgs ap = a;
             ap.rki_all = h->d_rki_all;
             ap.sun_all = h->d_sun_all;
-            CK(h->ops->chem_queue(ap, q, h->q_sync, h->q_wpb, h->q_nblocks, s));
+            if (coop) {
+                // as few cells per block as keep every SM busy: the cells of an SM share its FP64 pipe
+                const int cells = (int)std::min<long long>(h->ops->coop_max_cells, (n + h->nsm - 1) / h->nsm);
+                const int nb = (int)std::min<long long>(h->nsm, (n + cells - 1) / cells);
+                CK(h->ops->chem_coop(ap, q, cells, nb, s));
+            } else {
+                CK(h->ops->chem_queue(ap, q, h->q_sync, h->q_wpb, h->q_nblocks, s));
+            }
         } else {
             CK(h->ops->chem_queue(a, q, h->q_sync, h->q_wpb, h->q_nblocks, s));
         }

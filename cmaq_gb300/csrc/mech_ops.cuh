@@ -9,6 +9,7 @@
 #include "adjoint.cuh"
 #include "ddm.cuh"
 #include "gear.cuh"
+#include "coop.cuh"
 
 struct MechOps {
     const char* name;
@@ -51,6 +52,11 @@ struct MechOps {
     cudaError_t (*gear_warp)(const chem::GridArgs&, const chem::QueueArgs&, const chem::GearArgs&, bool grid,
                              int nblocks, cudaStream_t);
     cudaError_t (*gear_warp_occupancy)(int* blocks_per_sm);
+    // cooperative ROS3: one cell per warp, `cells` warps per block; taken for calls of at most
+    // coop_limit cells
+    int coop_max_cells;
+    long long coop_limit;
+    cudaError_t (*chem_coop)(const chem::GridArgs&, const chem::QueueArgs&, int cells, int nblocks, cudaStream_t);
 };
 
 #define DEFINE_MECH_OPS(NS, SYMBOL)                                                                 \
@@ -220,6 +226,15 @@ struct MechOps {
         *bps = a < b ? a : b;                                                                       \
         return r;                                                                                   \
     }                                                                                               \
+    cudaError_t chem_coop_(const chem::GridArgs& a, const chem::QueueArgs& q, int cells, int nb, cudaStream_t s) \
+    {                                                                                               \
+        const size_t bytes = coop::smem_bytes<NS::Coop>(cells);                                     \
+        cudaError_t r = cudaFuncSetAttribute(coop::k_chem_ros3_coop<T_, NS::Coop>,                  \
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); \
+        if (r != cudaSuccess) return r;                                                             \
+        coop::k_chem_ros3_coop<T_, NS::Coop><<<nb, cells * 32, bytes, s>>>(a, q);                   \
+        return cudaGetLastError();                                                                  \
+    }                                                                                               \
     cudaError_t occupancy_(int* bps)                                                                \
     {                                                                                               \
         int a = 0, b = 0;                                                                           \
@@ -240,4 +255,4 @@ struct MechOps {
                                    T_::EBI_DELTAT,                                                  \
                                    T_::ADJ_WS_ELEMS, adj_forward_, adj_reverse_, adj_occupancy_, ddm_update_,     \
                                    rconst_, rconst_pass_, occupancy_, T_::GEAR_WS_ELEMS, gear_, gear_occupancy_, \
-                                   gear_warp_, gear_warp_occupancy_};
+                                   gear_warp_, gear_warp_occupancy_, NS::Coop::MAX_CELLS, NS::COOP_LIMIT, chem_coop_};

@@ -432,6 +432,8 @@ def write_outputs(cmaq_root: str, mech: str, out_root: Path = REPO) -> dict:
     for fname, text in cuda_sources(m, prog, sp, mech, src_hash, ebi_decl).items():
         (cdir / fname).write_text(text)
     (cdir / f"{mech}_ebi.cu").write_text(ebi_tu)
+    from .coop import write as write_coop
+    write_coop(mech, cdir)   # reads the manifest written above (of the package: out_root may differ)
     return man
 
 

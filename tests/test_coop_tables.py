@@ -1,0 +1,103 @@
+"""The lane schedules of the cooperative kernels (mechgen/coop.py) against the sequential
+operations, on the CPU: both are carried out on expressions instead of numbers, the
+schedule from its encoded rows with the kernel's visibility of stores, and every element must
+end as the same expression (the same operations on the same values in the same order).
+"""
+import pytest
+
+from cmaq_gb300.mechgen import coop as C
+
+
+class Terms:
+    """Expressions by number: equal operations on equal operands have equal numbers."""
+
+    def __init__(self):
+        self.ids = {}
+
+    def __call__(self, *key):
+        return self.ids.setdefault(key, len(self.ids))
+
+
+def sequential(ops, start, term):
+    x = dict(start)
+    for kind, d, a, b, neg, init in ops:
+        if kind == "D":
+            x[d] = term("rcp", x[d])
+            continue
+        vb = term("const", b[1]) if isinstance(b, tuple) else x[b]
+        va = x[d] if init == C.MULACC else x[a]
+        x[d] = term("fma", neg, va, vb, x[d] if init == C.LOAD else "-0")
+    return x
+
+
+def rows_run(rows, start, consts, term):
+    """The kernel's loop: operands of row t + 2 loaded before the results of row t are stored."""
+    x = dict(start)
+    width = len(rows[0])
+    acc = [term("idle", ln) for ln in range(width)]
+
+    def load(row):
+        got = []
+        for w0, w1 in row:
+            a, b, d = (w0 & 0xfff8) // 8, (w0 >> 19) & 0x1fff, (w1 & 0xfff8) // 8
+            got.append((x[a], term("const", consts[b]) if w1 & C.B_CONST else x[b], x[d]))
+        return got
+
+    idle = [(0, 0)] * width
+    at = lambda t: load(rows[t] if t < len(rows) else idle)
+    ops, pending, recip = [at(0), at(1)], {}, False
+    for t, row in enumerate(rows):
+        if t % C.UNROLL == 0:
+            recip = bool(row[0][0] & C.A_RECIP)
+            if recip:                                      # a block of its own: the rest of it is not read
+                x.update(pending)
+                pending = {}
+                assert all(w0 & C.A_RECIP for w0, _ in row)
+                for w0, w1 in row:
+                    if w1 & C.D_STORE:
+                        x[(w1 & 0xfff8) // 8] = term("rcp", x[(w1 & 0xfff8) // 8])
+                ops = [at(t + C.UNROLL), at(t + C.UNROLL + 1)]
+        if recip:
+            continue
+        assert not any(w0 & C.A_RECIP for w0, _ in row)
+        cur, results = ops.pop(0), {}
+        for ln, (w0, w1) in enumerate(row):
+            a, b, c = cur[ln]
+            if w1 & C.C_KEEP and w1 & C.A_NEG and (w0 & 0xffff) == (w0 >> 16) == (w1 & 0xfff8):
+                continue                                   # idle lane: acc = -0 * 0 + acc
+            if not w1 & C.C_LOAD:
+                c = acc[ln] if w1 & C.C_KEEP else "-0"
+            if w1 & C.C_MULACC:
+                a = acc[ln]
+            acc[ln] = term("fma", bool(w1 & C.A_NEG), a, b, c)
+            if w1 & C.D_STORE:
+                d = (w1 & 0xfff8) // 8
+                assert d not in results
+                results[d] = acc[ln]
+        x.update(pending)                                  # row t - 1's results, then row t + 2's operands
+        pending = results
+        ops.append(at(t + 2))
+    x.update(pending)
+    return x
+
+
+@pytest.mark.parametrize("mech", ["cb6r5_ae7_aq", "cracmm2"])
+@pytest.mark.parametrize("width", [C.WIDTH, 8])
+def test_rows_carry_out_the_sequential_operations(mech, width):
+    m, sp = C.mechanism(mech)
+    lay, consts, tables = C.ros3_tables(mech, width)
+    for name, prog in C.ros3_programs(m, sp).items():
+        ops = lay.place(prog.ops)
+        term = Terms()
+        start = {e: term("in", e) for e in range(lay.elems)}
+        want = sequential(ops, start, term)
+        got = rows_run(tables[name], start, consts, term)
+        # partial-derivative products are scratch: elements that nothing reads any more
+        scratch = set(lay.alias.values()) if name == "stage1" else set()
+        assert all(got[e] == want[e] for e in range(lay.elems) if e not in scratch), name
+
+
+@pytest.mark.parametrize("mech", ["cb6r5_ae7_aq", "cracmm2"])
+def test_tables_are_the_generated_ones(mech):
+    for name, text in C.sources(mech).items():
+        assert (C.PKG / "csrc" / "gen" / name).read_text() == text
