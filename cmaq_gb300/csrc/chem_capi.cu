@@ -106,11 +106,11 @@ struct cmaqchem_handle {
     int q_nblocks = 0;
     int q_bps_cap = 0;       // blocks per SM of the queue kernel, 0: as many as fit
     int ebi_warp = 1;        // EBI: 1 one cell per warp (shared memory), 0 one cell per lane
-    int ebi_defer = 100;     // EBI: > 0 one cell per lane, cells past this many iterations per warp
-                             // (100 measured best of 20-800 on CB6r5: +10 % over warps alone)
+    int ebi_defer = 0;       // EBI: > 0 one cell per lane, cells past this many iterations per warp
+                             // (100, the best of 20-800, takes 491 and 885 ms where the warps alone
+                             // take 288 and 668 ms for 27,880 and 200,000 CB6r5 cells)
     int* d_ebi_def = nullptr;
     unsigned long long* d_ebi_ndef = nullptr;
-    int ebiw_nblocks = 0;
     size_t ws_warps = 0;     // workspace capacity in warps
     int ws_elems = 0;        // workspace elements per lane (the solver's layout)
     // SMVGEAR
@@ -375,10 +375,6 @@ extern "C" int cmaqchem_init(const cmaqchem_cfg* cfg, cmaqchem_handle** out)
             if (upload_gear_coef(h)) return -1;
         }
         if (cfg->solver == CMAQCHEM_SOLVER_EBI) {
-            int bw = 0;
-            CK(m->ebi_warp_occupancy(&bw));
-            h->ebiw_nblocks = h->nsm * (bw > 0 ? bw : 1);
-            if (ensure_ws(h, (size_t)h->ebiw_nblocks * chem::EBIW_WPB)) return -1;
             CK(cudaMalloc(&h->d_ebi_def, sizeof(int) * h->ncell));
             CK(cudaMalloc(&h->d_ebi_ndef, sizeof(unsigned long long)));
         }
@@ -403,8 +399,9 @@ extern "C" int cmaqchem_init(const cmaqchem_cfg* cfg, cmaqchem_handle** out)
         CK(cudaMalloc(&h->d_hist, sizeof(unsigned int) * chem::QUEUE_BINS));
         CK(cudaMalloc(&h->d_cursor, sizeof(unsigned long long) * chem::QUEUE_BINS));
         CK(cudaMalloc(&h->d_head, sizeof(unsigned long long)));
-        if (cfg->solver == CMAQCHEM_SOLVER_ROS3 &&
-            (cfg->schedule == CMAQCHEM_SCHED_QUEUE || use_coop(h, h->ncell))) {
+        if (cfg->solver == CMAQCHEM_SOLVER_EBI ||
+            (cfg->solver == CMAQCHEM_SOLVER_ROS3 &&
+             (cfg->schedule == CMAQCHEM_SCHED_QUEUE || use_coop(h, h->ncell)))) {
             // the rate-constant pass's arrays, when they leave a quarter of the free memory
             const size_t bytes = sizeof(double) * (size_t)m->nrxns * h->ncell;
             size_t free_b = 0, total_b = 0;
@@ -562,7 +559,25 @@ static int enqueue_step(cmaqchem_handle* h, const chem::GridArgs& a, int itmstep
             ebi::steps_for(itmstep, h->ops->ebi_deltat, &e.n_ebi_steps, &e.tmstep);
             e.fwd = h->d_ebi_fwd;
             e.rev = h->d_ebi_rev;
-            if (h->ebi_defer > 0) {
+            // the cells of [c0, c1), or those of a deferred list: one cell per warp, few to a block
+            auto by_warps = [&](const chem::QueueArgs& qw, const chem::EbiArgs& ew) -> int {
+                chem::GridArgs ap = a;
+                ap.rki_all = h->d_rki_all;
+                ap.sun_all = h->d_sun_all;
+                CK(h->ops->ebi_rconst_pass(a, c0, c1, h->d_rki_all, h->d_sun_all, h->nblocks, s));
+                // A call lasts at least as long as its slowest cell, whose iterations take longer
+                // the more warps share the SM: one per sub-partition up to 256 cells per SM (27,880
+                // CB6r5 cells: 288 ms with 4 warps, 347 with 8, 383 with 10), above that 8 (200,000
+                // cells: 1,064, 668 and 626 ms; a later call of the hour 212, 149 and 165 ms).
+                const long long share = (n + h->nsm - 1) / h->nsm;
+                const int cells = (int)std::min<long long>(share <= 256 ? 4 : std::min(8, h->ops->ebi_max_cells), share);
+                const int nb = (int)std::min<long long>(h->nsm, (n + cells - 1) / cells);
+                CK(h->ops->chem_ebi_warp(ap, qw, ew, cells, nb, s));
+                return 0;
+            };
+            if (!h->d_rki_all) {   // no room for the rates of the call: one cell per lane
+                CK(h->ops->chem_ebi(a, q, e, h->nblocks, s));
+            } else if (h->ebi_defer > 0) {
                 // one cell per lane for the cells that finish within ebi_defer iterations,
                 // then one cell per warp for the others
                 e.defer_after = h->ebi_defer;
@@ -574,9 +589,9 @@ static int enqueue_step(cmaqchem_handle* h, const chem::GridArgs& a, int itmstep
                 chem::EbiArgs e2 = e;
                 e2.defer_after = 0;
                 CK(cudaMemsetAsync(h->d_head, 0, sizeof(unsigned long long), s));
-                CK(h->ops->chem_ebi_warp(a, q2, e2, h->ebiw_nblocks, s));
+                if (by_warps(q2, e2)) return -1;
             } else if (h->ebi_warp) {
-                CK(h->ops->chem_ebi_warp(a, q, e, h->ebiw_nblocks, s));
+                if (by_warps(q, e)) return -1;
             } else {
                 CK(h->ops->chem_ebi(a, q, e, h->nblocks, s));
             }

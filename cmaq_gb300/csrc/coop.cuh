@@ -29,7 +29,7 @@ namespace coop {
 
 constexpr int UNROLL = 4, AHEAD = 3;
 // operation encoding of mechgen/coop.py: acc = +-a * b + c
-constexpr uint32_t A_RECIP = 1u, C_LOAD = 1u, C_KEEP = 2u, C_MULACC = 4u, D_STORE = 1u << 16, B_CONST = 1u << 17,
+constexpr uint32_t A_SPECIAL = 1u, C_LOAD = 1u, C_KEEP = 2u, C_MULACC = 4u, D_STORE = 1u << 16, B_CONST = 1u << 17,
                    A_NEG = 1u << 31;
 
 // Shared memory by its 32-bit addresses and predicated instructions: with generic pointers
@@ -56,29 +56,36 @@ __device__ __forceinline__ uint2 ldw(uint32_t p)
     return v;
 }
 
+// Waits, with a limit, for the phase of an mbarrier to complete.
+__device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t parity)
+{
+    uint32_t done = 0;
+    for (int tries = 0; !done && tries < 1 << 20; ++tries)
+        asm volatile("{ .reg .pred q; mbarrier.try_wait.parity.shared.b64 q, [%1], %2; selp.u32 %0, 1, 0, q; }"
+                     : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    return done != 0;
+}
+
 // The block's stream of table rows: chunks of CHUNK rows, fetched by one bulk copy each into
-// two buffers in shared memory that all warps read, in the order in which an attempt goes
-// through them (stage1, rhs, solve, solve, and again).  A warp that fetched its rows itself
-// waited for the L2 on every row.
+// two buffers in shared memory that all warps read, in the order of one pass through the
+// programs (C::chunk), and again.  A warp that fetched its rows itself waited for the L2 on
+// every row.
 template <class C>
 struct Stream {
     static constexpr int W = 32;
     static constexpr uint32_t BYTES = C::CHUNK * W * 8;
     static constexpr uint32_t PITCH = (C::CHUNK + AHEAD) * W * 8;   // rows of zeros end a buffer: looked ahead at only
-    static constexpr int N1 = (C::STAGE1_ROWS + C::CHUNK - 1) / C::CHUNK,
-                         N2 = (C::RHS_ROWS + C::CHUNK - 1) / C::CHUNK,
-                         N3 = (C::SOLVE_ROWS + C::CHUNK - 1) / C::CHUNK;
     uint32_t buf, bar;   // shared addresses: two buffers, two barriers
-    int k;               // chunk of the attempt, 0 .. N1 + N2 + 2 N3 - 1
+    int k;               // chunk of the pass
     uint32_t turn;       // chunks taken so far
     bool ok;             // false: a copy did not arrive (the wait gave up)
 
-    __device__ __forceinline__ static int wrap(int c) { return c >= N1 + N2 + 2 * N3 ? c - (N1 + N2 + 2 * N3) : c; }
+    __device__ __forceinline__ static int wrap(int c) { return c >= C::PASS ? c - C::PASS : c; }
 
-    // thread 0: the copy of the attempt's chunk c into buffer i
+    // thread 0: the copy of the pass's chunk c into buffer i
     __device__ __forceinline__ void fetch(int c, uint32_t i)
     {
-        const uint2* src = C::rows() + (size_t)(c < N1 + N2 + N3 ? c : c - N3) * (C::CHUNK * W);
+        const uint2* src = C::rows() + (size_t)C::chunk(c) * (C::CHUNK * W);
         asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" : : "r"(bar + 8 * i), "r"(BYTES) : "memory");
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                      : : "r"(buf + PITCH * i), "l"(src), "r"(BYTES), "r"(bar + 8 * i) : "memory");
@@ -108,12 +115,8 @@ struct Stream {
     // waits (with a limit) for the current chunk and returns its shared address
     __device__ __forceinline__ uint32_t wait()
     {
-        const uint32_t i = turn & 1u, parity = turn >> 1 & 1u;
-        uint32_t done = 0;
-        for (int tries = 0; !done && tries < 1 << 20; ++tries)
-            asm volatile("{ .reg .pred q; mbarrier.try_wait.parity.shared.b64 q, [%1], %2; selp.u32 %0, 1, 0, q; }"
-                         : "=r"(done) : "r"(bar + 8 * i), "r"(parity) : "memory");
-        if (!done) ok = false;
+        const uint32_t i = turn & 1u;
+        if (!wait_parity(bar + 8 * i, turn >> 1 & 1u)) ok = false;
         return buf + PITCH * i;
     }
 
@@ -138,6 +141,80 @@ struct Stream {
     }
 };
 
+// The rows of a one-warp block that goes through its programs by demand: begin names the
+// chunks to come, cancel drops those not taken.
+template <class C>
+struct Feed {
+    static constexpr int W = 32;
+    static constexpr uint32_t BYTES = C::CHUNK * W * 8, PITCH = (C::CHUNK + AHEAD) * W * 8;
+    uint32_t buf, bar, turn;
+    int next, end;       // chunk to take next, end of what was begun
+    bool ok;
+
+    __device__ __forceinline__ void fetch(int c, uint32_t i)
+    {
+        const uint2* src = C::rows() + (size_t)c * (C::CHUNK * W);
+        asm volatile("fence.proxy.async.shared::cta;" : : : "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" : : "r"(bar + 8 * i), "r"(BYTES) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     : : "r"(buf + PITCH * i), "l"(src), "r"(BYTES), "r"(bar + 8 * i) : "memory");
+    }
+
+    __device__ __forceinline__ void init(void* smem)
+    {
+        buf = (uint32_t)__cvta_generic_to_shared(smem);
+        bar = buf + 2 * PITCH;
+        turn = 0;
+        next = end = 0;
+        ok = true;
+        for (uint32_t j = threadIdx.x; j < 2 * AHEAD * W; j += W)
+            *(uint2*)((char*)smem + PITCH * (j / (AHEAD * W)) + BYTES + 8 * (j % (AHEAD * W))) = make_uint2(0u, 0u);
+        if (threadIdx.x == 0) {
+            asm volatile("mbarrier.init.shared.b64 [%0], 1;" : : "r"(bar) : "memory");
+            asm volatile("mbarrier.init.shared.b64 [%0], 1;" : : "r"(bar + 8) : "memory");
+            asm volatile("fence.mbarrier_init.release.cluster;" : : : "memory");
+        }
+        __syncwarp();
+    }
+
+    // chunks [c0, c1): the first two are on their way when it returns
+    __device__ __forceinline__ void begin(int c0, int c1)
+    {
+        next = c0;
+        end = c1;
+        __syncwarp();
+        if (threadIdx.x == 0) {
+            fetch(c0, turn & 1u);
+            if (c0 + 1 < c1) fetch(c0 + 1, (turn + 1) & 1u);
+        }
+    }
+
+    __device__ __forceinline__ uint32_t wait()
+    {
+        const uint32_t i = turn & 1u;
+        if (!wait_parity(bar + 8 * i, turn >> 1 & 1u)) ok = false;
+        return buf + PITCH * i;
+    }
+
+    __device__ __forceinline__ void release()
+    {
+        __syncwarp();
+        if (threadIdx.x == 0 && next + 2 < end) fetch(next + 2, turn & 1u);
+        ++turn;
+        ++next;
+    }
+
+    __device__ __forceinline__ void cancel()
+    {
+        for (int n = min(2, end - next); n > 0; --n) {
+            wait();
+            ++turn;
+        }
+        next = end = 0;
+        __syncwarp();
+    }
+};
+
 struct Operands {
     double a, b, c;
 };
@@ -151,18 +228,32 @@ __device__ __forceinline__ Operands operands(uint2 w, uint32_t cell, uint32_t cs
     return o;
 }
 
-static __device__ __noinline__ void recip_row(uint2 w, uint32_t cell)
+// A row of special operations (mechgen/coop.py); lanes without one have kind 0.
+static __device__ __noinline__ void special_row(uint2 w, uint32_t cell, uint32_t cst)
 {
-    const uint32_t p = cell + (w.y & 0xfff8u);
-    sts_if(p, w.y & D_STORE, fpdiv::div(1.0, lds_if(p, w.y & D_STORE, 1.0)));
+    enum { RCP = 1, DIV, SQRT, MAX, SIGN };
+    const uint32_t kind = w.y & 7u;
+    const double a = lds(cell + (w.x & 0xfff8u));
+    const double b = lds((w.y & B_CONST ? cst : cell) + (w.x >> 16));
+    double r = 0.0;
+    if (__any_sync(0xffffffffu, kind == RCP || kind == DIV)) {
+        const bool on = kind == RCP || kind == DIV;
+        r = fpdiv::div(kind == DIV ? a : 1.0, on ? b : 1.0);
+    }
+    __syncwarp();
+    if (kind == SQRT) r = sqrt(b);
+    if (kind == MAX) r = fmax(a, b);
+    if (kind == SIGN) r = copysign(1.0, b);
+    __syncwarp();   // every lane has read its operands
+    sts_if(cell + (w.y & 0xfff8u), w.y & D_STORE, r);
 }
 
-// The rows of a program on the warp's cell; every warp of the block calls it.  While row t's FMA is under way, row t - 1's results are stored and then the
+// The rows of a program on the warp's cell; every warp of the block calls it (S: Stream or Feed).  While row t's FMA is under way, row t - 1's results are stored and then the
 // operands of row t + 2 loaded, so that a row waits for neither (with the operands of row
 // t + 1 loaded there it waited for them: 135 cycles a row); the schedule knows that a row's
 // results can be loaded three rows later.
-template <class C>
-__device__ __forceinline__ void run(Stream<C>& st, int rows, uint32_t cell, uint32_t cst)
+template <class C, class S>
+__device__ __forceinline__ void run(S& st, int rows, uint32_t cell, uint32_t cst)
 {
     constexpr int W = 32;
     double acc = 0.0;
@@ -175,11 +266,11 @@ __device__ __forceinline__ void run(Stream<C>& st, int rows, uint32_t cell, uint
             uint2 w = ldw(p), w1 = ldw(p + W * 8), w2 = ldw(p + 2 * W * 8);
             Operands o = operands(w, cell, cst), o1 = operands(w1, cell, cst);
             for (int r = 0; r < nr; r += UNROLL) {   // programs are padded to a multiple of UNROLL rows
-                if (__any_sync(0xffffffffu, w.x & A_RECIP)) {   // all lanes or none
+                if (__any_sync(0xffffffffu, w.x & A_SPECIAL)) {   // all lanes or none
                     sts_if(cell + (pending & 0xfff8u), pending & D_STORE, acc);
                     pending = 0;
                     __syncwarp();
-                    recip_row(w, cell);
+                    special_row(w, cell, cst);
                     __syncwarp();
                     p += UNROLL * W * 8;
                     w = ldw(p);

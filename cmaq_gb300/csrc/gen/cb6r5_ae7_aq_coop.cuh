@@ -1,17 +1,45 @@
-// Generated by cmaq_gb300.mechgen.coop from mechs/cb6r5_ae7_aq/manifest.json.  Do not edit.
-// Sizes and tables of the cooperative ROS3 kernel (csrc/coop.cuh).
+// Generated by cmaq_gb300.mechgen.coop from mechs/cb6r5_ae7_aq/manifest.json and gen/cb6r5_ae7_aq_ebi.cu.  Do not edit.
+// Sizes and tables of the cooperative kernels (csrc/coop.cuh, csrc/ebi_coop.cuh).
 #pragma once
 #include <cuda_runtime.h>
 namespace mech_cb6r5_ae7_aq {
 extern __device__ const double c_coop_const[264];
 extern __device__ const uint2 c_coop_rows[38528];
+extern __device__ const double c_coopebi_const[264];
+extern __device__ const uint2 c_coopebi_rows[8960];
+extern __device__ const double c_coopgear_const[264];
+extern __device__ const uint2 c_coopgear_rows[29184];
 struct Coop {
     static constexpr int ELEMS = 3223, NCONST = 264, MAX_CELLS = 8;
-    static constexpr int Y = 0, V = 149, K1 = 298, K2 = 447, T = 596;
-    static constexpr int RKI = 745, G = 3132, Z = 3133;
+    static constexpr int Y = 0, V = 149, K1 = 298, K2 = 447, T = 596, RKI = 745, G = 3132, Z = 3133;
     static constexpr int CHUNK = 28, TABLE_SMEM = 15936;
+    static constexpr int STAGE1_ROWS = 708, RHS_ROWS = 172, SOLVE_ROWS = 280;
+    // chunks of one pass through the programs (stage1, rhs, solve, solve), and where each lies
+    static constexpr int PASS = 53;
+    static __device__ __forceinline__ int chunk(int k) { return k < 43 ? k : k - 10; }
     static __device__ __forceinline__ const double* constants() { return c_coop_const; }
     static __device__ __forceinline__ const uint2* rows() { return c_coop_rows; }
-    static constexpr int STAGE1_ROWS = 708, RHS_ROWS = 172, SOLVE_ROWS = 280;
+};
+struct CoopEbi {
+    static constexpr int ELEMS = 2464, NCONST = 264, MAX_CELLS = 10;
+    static constexpr int YC = 0, YC0 = 149, YCP = 298, PROD = 447, LOSS = 596, PNEG = 745, RKI = 894, DTC = 1592, Z = 1593, ONE = 1594;
+    static constexpr int CHUNK = 28, TABLE_SMEM = 15936;
+    static constexpr int ITERATION_ROWS = 256;
+    // chunks of one pass through the programs (iteration), and where each lies
+    static constexpr int PASS = 10;
+    static __device__ __forceinline__ int chunk(int k) { return k; }
+    static __device__ __forceinline__ const double* constants() { return c_coopebi_const; }
+    static __device__ __forceinline__ const uint2* rows() { return c_coopebi_rows; }
+};
+struct CoopGear {
+    static constexpr int ELEMS = 5312, NCONST = 264, MAX_CELLS = 5;
+    static constexpr int Q = 4120, R1 = 0, Z = 1, ONE = 2, WORKSPACE = 4;
+    static constexpr int CHUNK = 16, TABLE_SMEM = 9792;
+    static constexpr int PREDICTOR_ROWS = 440, RHS_ROWS = 168, SOLVE_ROWS = 280;
+    // chunks of one pass through the programs (predictor, rhs, solve), and where each lies
+    static constexpr int PASS = 57;
+    static __device__ __forceinline__ int chunk(int k) { return k; }
+    static __device__ __forceinline__ const double* constants() { return c_coopgear_const; }
+    static __device__ __forceinline__ const uint2* rows() { return c_coopgear_rows; }
 };
 }  // namespace mech_cb6r5_ae7_aq

@@ -83,16 +83,6 @@ constexpr int GEAR_CONC = 4265;
 constexpr int GEAR_E = 149;
 constexpr int GEAR_CAVEG = 2277;
 constexpr int GEAR_CFINI = 5159;
-constexpr int EBIW_YC = 0;
-constexpr int EBIW_YC0 = 149;
-constexpr int EBIW_YCP = 298;
-constexpr int EBIW_PROD = 447;
-constexpr int EBIW_LOSS = 596;
-constexpr int EBIW_PNEG = 745;
-constexpr int EBIW_NOTMAX = 894;
-constexpr int EBIW_RKI = 1043;
-constexpr int EBIW_RXRAT = 1392;
-constexpr int EBIW_ELEMS = 1741;
 constexpr double FLOPS_STEP_DAY = 36947.0;
 constexpr double FLOPS_STEP_NIGHT = 34766.0;
 extern __constant__ int c_inew2old[149];
@@ -330,24 +320,6 @@ __device__ void ebi_hrg1(double* __restrict__ ws, double dtc);
 __device__ void ebi_hrg2(double* __restrict__ ws, double dtc);
 __device__ void ebi_hrg3(double* __restrict__ ws, double dtc);
 __device__ void ebi_hrg4(double* __restrict__ ws, double dtc);
-constexpr int EBIW_NRATE = 328;
-constexpr int EBIW_NPL = 273;
-constexpr int EBIW_NTERM = 1109;
-extern __device__ const int c_ebiw_rate_r[EBIW_NRATE];
-extern __device__ const int c_ebiw_rate_nf[EBIW_NRATE];
-extern __device__ const int c_ebiw_rate_sp[EBIW_NRATE * 3];
-extern __device__ const int c_ebiw_pl_ptr[33];
-extern __device__ const int c_ebiw_pl_kind[EBIW_NPL];
-extern __device__ const int c_ebiw_pl_sp[EBIW_NPL];
-extern __device__ const int c_ebiw_pl_t0[EBIW_NPL + 1];
-extern __device__ const int c_ebiw_term_r[EBIW_NTERM > 0 ? EBIW_NTERM : 1];
-extern __device__ const double c_ebiw_term_c[EBIW_NTERM > 0 ? EBIW_NTERM : 1];
-namespace wsm {
-__device__ void ebi_hrg1(double* __restrict__ sm, double dtc);
-__device__ void ebi_hrg2(double* __restrict__ sm, double dtc);
-__device__ void ebi_hrg3(double* __restrict__ sm, double dtc);
-__device__ void ebi_hrg4(double* __restrict__ sm, double dtc);
-}  // namespace wsm
 __device__ __forceinline__ void gear_pdecomp_0(double* __restrict__ ws, double r1delt)
 {
     gear_pdecomp_0_0(ws, r1delt);
@@ -762,16 +734,6 @@ struct Traits {
     static constexpr int GEAR_E = mech_cb6r5_ae7_aq::GEAR_E;
     static constexpr int GEAR_CAVEG = mech_cb6r5_ae7_aq::GEAR_CAVEG;
     static constexpr int GEAR_CFINI = mech_cb6r5_ae7_aq::GEAR_CFINI;
-    static constexpr int EBIW_YC = mech_cb6r5_ae7_aq::EBIW_YC;
-    static constexpr int EBIW_YC0 = mech_cb6r5_ae7_aq::EBIW_YC0;
-    static constexpr int EBIW_YCP = mech_cb6r5_ae7_aq::EBIW_YCP;
-    static constexpr int EBIW_PROD = mech_cb6r5_ae7_aq::EBIW_PROD;
-    static constexpr int EBIW_LOSS = mech_cb6r5_ae7_aq::EBIW_LOSS;
-    static constexpr int EBIW_PNEG = mech_cb6r5_ae7_aq::EBIW_PNEG;
-    static constexpr int EBIW_NOTMAX = mech_cb6r5_ae7_aq::EBIW_NOTMAX;
-    static constexpr int EBIW_RKI = mech_cb6r5_ae7_aq::EBIW_RKI;
-    static constexpr int EBIW_RXRAT = mech_cb6r5_ae7_aq::EBIW_RXRAT;
-    static constexpr int EBIW_ELEMS = mech_cb6r5_ae7_aq::EBIW_ELEMS;
     static constexpr const char* name() { return mech_cb6r5_ae7_aq::NAME; }
     static __device__ __forceinline__ int iold2new(int s) { return mech_cb6r5_ae7_aq::c_iold2new[s]; }
     static __device__ __forceinline__ int inew2old(int i) { return mech_cb6r5_ae7_aq::c_inew2old[i]; }
@@ -809,23 +771,9 @@ struct Traits {
     static __device__ __forceinline__ void ebi_hrrates(double* ws) { mech_cb6r5_ae7_aq::ebi_hrrates(ws); }
     static __device__ __forceinline__ void ebi_hrprodloss(double* ws) { mech_cb6r5_ae7_aq::ebi_hrprodloss(ws); }
     static __device__ __forceinline__ void ebi_hrg1(double* ws, double dtc) { mech_cb6r5_ae7_aq::ebi_hrg1(ws, dtc); }
-    static __device__ __forceinline__ void ebiw_hrg1(double* sm, double dtc) { mech_cb6r5_ae7_aq::wsm::ebi_hrg1(sm, dtc); }
     static __device__ __forceinline__ void ebi_hrg2(double* ws, double dtc) { mech_cb6r5_ae7_aq::ebi_hrg2(ws, dtc); }
-    static __device__ __forceinline__ void ebiw_hrg2(double* sm, double dtc) { mech_cb6r5_ae7_aq::wsm::ebi_hrg2(sm, dtc); }
     static __device__ __forceinline__ void ebi_hrg3(double* ws, double dtc) { mech_cb6r5_ae7_aq::ebi_hrg3(ws, dtc); }
-    static __device__ __forceinline__ void ebiw_hrg3(double* sm, double dtc) { mech_cb6r5_ae7_aq::wsm::ebi_hrg3(sm, dtc); }
     static __device__ __forceinline__ void ebi_hrg4(double* ws, double dtc) { mech_cb6r5_ae7_aq::ebi_hrg4(ws, dtc); }
-    static __device__ __forceinline__ void ebiw_hrg4(double* sm, double dtc) { mech_cb6r5_ae7_aq::wsm::ebi_hrg4(sm, dtc); }
-    static constexpr int EBIW_NRATE = mech_cb6r5_ae7_aq::EBIW_NRATE;
-    static __device__ __forceinline__ const int* ebiw_rate_r() { return mech_cb6r5_ae7_aq::c_ebiw_rate_r; }
-    static __device__ __forceinline__ const int* ebiw_rate_nf() { return mech_cb6r5_ae7_aq::c_ebiw_rate_nf; }
-    static __device__ __forceinline__ const int* ebiw_rate_sp() { return mech_cb6r5_ae7_aq::c_ebiw_rate_sp; }
-    static __device__ __forceinline__ const int* ebiw_pl_ptr() { return mech_cb6r5_ae7_aq::c_ebiw_pl_ptr; }
-    static __device__ __forceinline__ const int* ebiw_pl_kind() { return mech_cb6r5_ae7_aq::c_ebiw_pl_kind; }
-    static __device__ __forceinline__ const int* ebiw_pl_sp() { return mech_cb6r5_ae7_aq::c_ebiw_pl_sp; }
-    static __device__ __forceinline__ const int* ebiw_pl_t0() { return mech_cb6r5_ae7_aq::c_ebiw_pl_t0; }
-    static __device__ __forceinline__ const int* ebiw_term_r() { return mech_cb6r5_ae7_aq::c_ebiw_term_r; }
-    static __device__ __forceinline__ const double* ebiw_term_c() { return mech_cb6r5_ae7_aq::c_ebiw_term_c; }
     static constexpr int GW_NACT = 349;
     static constexpr int GW_NEX = 268;
     static constexpr int GW_NFL = 22;

@@ -83,16 +83,6 @@ constexpr int GEAR_CONC = 6958;
 constexpr int GEAR_E = 189;
 constexpr int GEAR_CAVEG = 3295;
 constexpr int GEAR_CFINI = 8092;
-constexpr int EBIW_YC = 0;
-constexpr int EBIW_YC0 = 189;
-constexpr int EBIW_YCP = 378;
-constexpr int EBIW_PROD = 567;
-constexpr int EBIW_LOSS = 756;
-constexpr int EBIW_PNEG = 945;
-constexpr int EBIW_NOTMAX = 1134;
-constexpr int EBIW_RKI = 1323;
-constexpr int EBIW_RXRAT = 1854;
-constexpr int EBIW_ELEMS = 2385;
 constexpr double FLOPS_STEP_DAY = 79988.0;
 constexpr double FLOPS_STEP_NIGHT = 77148.0;
 extern __constant__ int c_inew2old[189];
@@ -462,24 +452,6 @@ __device__ void ebi_hrg1(double* __restrict__ ws, double dtc);
 __device__ void ebi_hrg2(double* __restrict__ ws, double dtc);
 __device__ void ebi_hrg3(double* __restrict__ ws, double dtc);
 __device__ void ebi_hrg4(double* __restrict__ ws, double dtc);
-constexpr int EBIW_NRATE = 510;
-constexpr int EBIW_NPL = 352;
-constexpr int EBIW_NTERM = 2196;
-extern __device__ const int c_ebiw_rate_r[EBIW_NRATE];
-extern __device__ const int c_ebiw_rate_nf[EBIW_NRATE];
-extern __device__ const int c_ebiw_rate_sp[EBIW_NRATE * 3];
-extern __device__ const int c_ebiw_pl_ptr[33];
-extern __device__ const int c_ebiw_pl_kind[EBIW_NPL];
-extern __device__ const int c_ebiw_pl_sp[EBIW_NPL];
-extern __device__ const int c_ebiw_pl_t0[EBIW_NPL + 1];
-extern __device__ const int c_ebiw_term_r[EBIW_NTERM > 0 ? EBIW_NTERM : 1];
-extern __device__ const double c_ebiw_term_c[EBIW_NTERM > 0 ? EBIW_NTERM : 1];
-namespace wsm {
-__device__ void ebi_hrg1(double* __restrict__ sm, double dtc);
-__device__ void ebi_hrg2(double* __restrict__ sm, double dtc);
-__device__ void ebi_hrg3(double* __restrict__ sm, double dtc);
-__device__ void ebi_hrg4(double* __restrict__ sm, double dtc);
-}  // namespace wsm
 __device__ __forceinline__ void gear_pdecomp_0(double* __restrict__ ws, double r1delt)
 {
     gear_pdecomp_0_0(ws, r1delt);
@@ -1126,16 +1098,6 @@ struct Traits {
     static constexpr int GEAR_E = mech_cracmm2::GEAR_E;
     static constexpr int GEAR_CAVEG = mech_cracmm2::GEAR_CAVEG;
     static constexpr int GEAR_CFINI = mech_cracmm2::GEAR_CFINI;
-    static constexpr int EBIW_YC = mech_cracmm2::EBIW_YC;
-    static constexpr int EBIW_YC0 = mech_cracmm2::EBIW_YC0;
-    static constexpr int EBIW_YCP = mech_cracmm2::EBIW_YCP;
-    static constexpr int EBIW_PROD = mech_cracmm2::EBIW_PROD;
-    static constexpr int EBIW_LOSS = mech_cracmm2::EBIW_LOSS;
-    static constexpr int EBIW_PNEG = mech_cracmm2::EBIW_PNEG;
-    static constexpr int EBIW_NOTMAX = mech_cracmm2::EBIW_NOTMAX;
-    static constexpr int EBIW_RKI = mech_cracmm2::EBIW_RKI;
-    static constexpr int EBIW_RXRAT = mech_cracmm2::EBIW_RXRAT;
-    static constexpr int EBIW_ELEMS = mech_cracmm2::EBIW_ELEMS;
     static constexpr const char* name() { return mech_cracmm2::NAME; }
     static __device__ __forceinline__ int iold2new(int s) { return mech_cracmm2::c_iold2new[s]; }
     static __device__ __forceinline__ int inew2old(int i) { return mech_cracmm2::c_inew2old[i]; }
@@ -1173,23 +1135,9 @@ struct Traits {
     static __device__ __forceinline__ void ebi_hrrates(double* ws) { mech_cracmm2::ebi_hrrates(ws); }
     static __device__ __forceinline__ void ebi_hrprodloss(double* ws) { mech_cracmm2::ebi_hrprodloss(ws); }
     static __device__ __forceinline__ void ebi_hrg1(double* ws, double dtc) { mech_cracmm2::ebi_hrg1(ws, dtc); }
-    static __device__ __forceinline__ void ebiw_hrg1(double* sm, double dtc) { mech_cracmm2::wsm::ebi_hrg1(sm, dtc); }
     static __device__ __forceinline__ void ebi_hrg2(double* ws, double dtc) { mech_cracmm2::ebi_hrg2(ws, dtc); }
-    static __device__ __forceinline__ void ebiw_hrg2(double* sm, double dtc) { mech_cracmm2::wsm::ebi_hrg2(sm, dtc); }
     static __device__ __forceinline__ void ebi_hrg3(double* ws, double dtc) { mech_cracmm2::ebi_hrg3(ws, dtc); }
-    static __device__ __forceinline__ void ebiw_hrg3(double* sm, double dtc) { mech_cracmm2::wsm::ebi_hrg3(sm, dtc); }
     static __device__ __forceinline__ void ebi_hrg4(double* ws, double dtc) { mech_cracmm2::ebi_hrg4(ws, dtc); }
-    static __device__ __forceinline__ void ebiw_hrg4(double* sm, double dtc) { mech_cracmm2::wsm::ebi_hrg4(sm, dtc); }
-    static constexpr int EBIW_NRATE = mech_cracmm2::EBIW_NRATE;
-    static __device__ __forceinline__ const int* ebiw_rate_r() { return mech_cracmm2::c_ebiw_rate_r; }
-    static __device__ __forceinline__ const int* ebiw_rate_nf() { return mech_cracmm2::c_ebiw_rate_nf; }
-    static __device__ __forceinline__ const int* ebiw_rate_sp() { return mech_cracmm2::c_ebiw_rate_sp; }
-    static __device__ __forceinline__ const int* ebiw_pl_ptr() { return mech_cracmm2::c_ebiw_pl_ptr; }
-    static __device__ __forceinline__ const int* ebiw_pl_kind() { return mech_cracmm2::c_ebiw_pl_kind; }
-    static __device__ __forceinline__ const int* ebiw_pl_sp() { return mech_cracmm2::c_ebiw_pl_sp; }
-    static __device__ __forceinline__ const int* ebiw_pl_t0() { return mech_cracmm2::c_ebiw_pl_t0; }
-    static __device__ __forceinline__ const int* ebiw_term_r() { return mech_cracmm2::c_ebiw_term_r; }
-    static __device__ __forceinline__ const double* ebiw_term_c() { return mech_cracmm2::c_ebiw_term_c; }
     static constexpr int GW_NACT = 531;
     static constexpr int GW_NEX = 455;
     static constexpr int GW_NFL = 29;

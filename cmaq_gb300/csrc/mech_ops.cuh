@@ -10,6 +10,7 @@
 #include "ddm.cuh"
 #include "gear.cuh"
 #include "coop.cuh"
+#include "ebi_coop.cuh"
 
 struct MechOps {
     const char* name;
@@ -30,9 +31,12 @@ struct MechOps {
     cudaError_t (*chem_ebi)(const chem::GridArgs&, const chem::QueueArgs&, const chem::EbiArgs&, int nblocks,
                             cudaStream_t);
     cudaError_t (*ebi_solve)(const chem::EbiSolveArgs&, int nblocks, cudaStream_t);
-    cudaError_t (*chem_ebi_warp)(const chem::GridArgs&, const chem::QueueArgs&, const chem::EbiArgs&, int nblocks,
-                                 cudaStream_t);
-    cudaError_t (*ebi_warp_occupancy)(int* blocks_per_sm);
+    // one cell per warp, `cells` warps per block (rates from ebi_rconst_pass)
+    int ebi_max_cells;
+    cudaError_t (*chem_ebi_warp)(const chem::GridArgs&, const chem::QueueArgs&, const chem::EbiArgs&, int cells,
+                                 int nblocks, cudaStream_t);
+    cudaError_t (*ebi_rconst_pass)(const chem::GridArgs&, long long c0, long long c1, double* rki, uint8_t* sunlit,
+                                   int nblocks, cudaStream_t);
     double ebi_deltat;
     int adj_ws_elems;
     cudaError_t (*adj_forward)(const adj::Args&, int nblocks, cudaStream_t);
@@ -117,29 +121,21 @@ struct MechOps {
         chem::k_chem_ebi_queue<T_><<<nb, chem::THREADS_PER_BLOCK, 0, s>>>(a, q, e);                 \
         return cudaGetLastError();                                                                  \
     }                                                                                               \
-    size_t ebiw_smem_() { return (size_t)chem::EBIW_WPB * T_::EBIW_ELEMS * sizeof(double); }        \
-    cudaError_t ebiw_attr_()                                                                        \
-    {                                                                                               \
-        cudaError_t r = cudaFuncSetAttribute(chem::k_chem_ebi_warp<T_>,                             \
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ebiw_smem_()); \
-        if (r != cudaSuccess) return r;                                                             \
-        return cudaFuncSetAttribute(chem::k_chem_ebi_warp<T_>, cudaFuncAttributePreferredSharedMemoryCarveout, \
-                                    (int)cudaSharedmemCarveoutMaxShared);                           \
-    }                                                                                               \
     cudaError_t chem_ebi_warp_(const chem::GridArgs& a, const chem::QueueArgs& q, const chem::EbiArgs& e, \
-                               int nb, cudaStream_t s)                                              \
+                               int cells, int nb, cudaStream_t s)                                   \
     {                                                                                               \
-        cudaError_t r = ebiw_attr_();                                                               \
+        const size_t bytes = coop::smem_bytes<NS::CoopEbi>(cells);                                  \
+        cudaError_t r = cudaFuncSetAttribute(chem::k_chem_ebi_warp<T_, NS::CoopEbi>,                \
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); \
         if (r != cudaSuccess) return r;                                                             \
-        chem::k_chem_ebi_warp<T_><<<nb, chem::EBIW_WPB * 32, ebiw_smem_(), s>>>(a, q, e);           \
+        chem::k_chem_ebi_warp<T_, NS::CoopEbi><<<nb, cells * 32, bytes, s>>>(a, q, e);              \
         return cudaGetLastError();                                                                  \
     }                                                                                               \
-    cudaError_t ebi_warp_occupancy_(int* bps)                                                       \
+    cudaError_t ebi_rconst_pass_(const chem::GridArgs& a, long long c0, long long c1, double* rki, uint8_t* sun, \
+                                 int nb, cudaStream_t s)                                            \
     {                                                                                               \
-        cudaError_t r = ebiw_attr_();                                                               \
-        if (r != cudaSuccess) return r;                                                             \
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, chem::k_chem_ebi_warp<T_>,        \
-                                                             chem::EBIW_WPB * 32, ebiw_smem_());    \
+        chem::k_ebi_rconst_pass<T_><<<nb, chem::THREADS_PER_BLOCK, 0, s>>>(a, c0, c1, rki, sun);    \
+        return cudaGetLastError();                                                                  \
     }                                                                                               \
     cudaError_t ebi_solve_(const chem::EbiSolveArgs& a, int nb, cudaStream_t s)                     \
     {                                                                                               \
@@ -251,7 +247,7 @@ struct MechOps {
                                    NS::FLOPS_STEP_DAY, NS::FLOPS_STEP_NIGHT,                        \
                                    NS::h_cgrid_index, NS::h_convert, NS::h_molwt, NS::h_inew2old,   \
                                    NS::h_iold2new, chem_static_, chem_queue_, queue_occupancy_,     \
-                                   solve_, chem_ebi_, ebi_solve_, chem_ebi_warp_, ebi_warp_occupancy_, \
+                                   solve_, chem_ebi_, ebi_solve_, NS::CoopEbi::MAX_CELLS, chem_ebi_warp_, ebi_rconst_pass_, \
                                    T_::EBI_DELTAT,                                                  \
                                    T_::ADJ_WS_ELEMS, adj_forward_, adj_reverse_, adj_occupancy_, ddm_update_,     \
                                    rconst_, rconst_pass_, occupancy_, T_::GEAR_WS_ELEMS, gear_, gear_occupancy_, \

@@ -2,8 +2,8 @@
 
 A routine of the cell's solver (rates, right-hand side, Jacobian, factorisation, triangular
 solves) is written down as the sequence of its scalar operations, every one of the form
-``acc = +-x[a] * x[b] + c`` or ``x[d] = 1 / x[d]``, in the order of the generated sequential
-code.  `schedule` deals these operations out to W lanes, row by row: a row is one operation
+``acc = +-x[a] * x[b] + c`` or a special one (quotient, square root, maximum, sign), in the
+order of the generated sequential code.  `schedule` deals these operations out to W lanes, row by row: a row is one operation
 per lane, and an operation is placed as soon as the values that it reads are there, longest
 remaining chain first.  No operation is changed and no sum is reordered: each element of the
 cell's state goes through the same operations on the same values as in the sequential
@@ -12,8 +12,8 @@ routine, so the results have the same bits.
 The kernel (csrc/coop.cuh) loads the operands of row t + 2 before it stores the results of
 row t, so a value is read at the earliest three rows after the one that computed it, unless
 the same lane goes on with it in its accumulator.  The kernel goes through UNROLL rows
-without a branch (a test for reciprocals in each row took 50 of its 165 cycles); a row of
-reciprocals takes the place of such a block.
+without a branch (a test for special rows in each row took 50 of its 165 cycles); a row of
+special operations takes the place of such a block.
 
 Tables are made from the mechanism's manifest alone:
 
@@ -22,11 +22,13 @@ Tables are made from the mechanism's manifest alone:
 from __future__ import annotations
 
 import json
+import math
+import re
 from dataclasses import dataclass, field
 from pathlib import Path
 
 from .emit_common import c_double
-from .emit_cuda import _jac_terms
+from .emit_cuda import Layout, _jac_terms
 from .fortran_tables import Mechanism
 from .sparse import SparseMech, build_sparse
 
@@ -34,33 +36,36 @@ PKG = Path(__file__).resolve().parents[1]
 VISIBLE = 3          # rows from the one that computes a value to the first that may load it
 CHUNK = 28           # rows of a table that are fetched together (more would cost CRACMM2 a cell)
 AHEAD = 3            # rows past a chunk's end whose words the kernel may look at
-UNROLL = 4           # rows that the kernel goes through without a branch: a row of reciprocals
-                     # comes only after a multiple of it, in a block of its own
-SLACK = 3            # how much shorter a reciprocal's chain may be than the longest one
+UNROLL = 4           # rows that the kernel goes through without a branch: a row of special
+                     # operations comes only after a multiple of it, in a block of its own
+SLACK = 3            # how much shorter a special operation's chain may be than the longest one
 SMEM_MAX = 227 * 1024
 TABLE_SMEM = 2 * (CHUNK + AHEAD) * 32 * 8 + 64   # two chunks in flight, each with rows of zeros, and their barriers
 
 # where an operation's addend comes from: the element itself, the lane's accumulator, -0.0
 # (the exact identity of an addition: a product alone); MULACC: acc * x[b]
 LOAD, KEEP, NEG0, MULACC = range(4)
+# special operations: 1 / x[b], x[a] / x[b], sqrt(x[b]), fmax(x[a], x[b]), copysign(1, x[b])
+RCP, DIV, SQRT, MAX, SIGN = range(1, 6)
 # encoding: word 0 = offset of a | offset of b << 16, word 1 = offset of d, and flags.
 # Offsets are bytes (multiples of 8) into the cell's state; b may be a constant's offset.
-A_RECIP, C_LOAD, C_KEEP, C_MULACC = 1, 1, 2, 4
+# Word 1 of a special operation (A_SPECIAL in word 0) holds its kind in place of the addend's.
+A_SPECIAL, C_LOAD, C_KEEP, C_MULACC = 1, 1, 2, 4
 D_STORE, B_CONST, A_NEG = 1 << 16, 1 << 17, 1 << 31
 ADDEND = {LOAD: C_LOAD, KEEP: C_KEEP, NEG0: 0, MULACC: C_MULACC}
 
 
 @dataclass
 class Program:
-    """Operations in sequential order: ("F", d, a, b, negate a, addend) or ("D", d).  Elements are
-    names or ("c", value) constants."""
+    """Operations in sequential order: ("F", d, a, b, negate a, addend) or ("D", d, a, b, False,
+    special kind).  Elements are names; b may be a ("c", value) constant."""
     ops: list = field(default_factory=list)
 
     def fma(self, d, a, b, neg=False, init=LOAD):
         self.ops.append(("F", d, a, b, neg, init))
 
-    def recip(self, d):
-        self.ops.append(("D", d, d, None, False, LOAD))
+    def special(self, kind, d, a, b):
+        self.ops.append(("D", d, a, b, False, kind))
 
 
 def dependencies(ops) -> list[list[tuple[int, str]]]:
@@ -70,9 +75,8 @@ def dependencies(ops) -> list[list[tuple[int, str]]]:
     for i, (kind, d, a, b, _, init) in enumerate(ops):
         p = []
         scaled = kind == "F" and init == NEG0 and a == d      # d = d * x[b]
-        reads = [d] if kind == "D" else ([b] if init == MULACC or scaled else [a, b])
-        for e in reads:
-            if isinstance(e, tuple):
+        for e in [b] if kind == "F" and init == MULACC or scaled else [a, b]:
+            if e is None or isinstance(e, tuple):
                 continue
             if e in last:
                 p.append((last[e], "R"))
@@ -99,7 +103,7 @@ class Schedule:
     store: list         # whether the operation's result goes to its element
 
 
-def schedule(ops, width: int, recip_cost: int = 3) -> Schedule:
+def schedule(ops, width: int, special_cost: int = 3) -> Schedule:
     """List scheduling, the longest remaining dependence chain first."""
     n = len(ops)
     preds = dependencies(ops)
@@ -120,7 +124,7 @@ def schedule(ops, width: int, recip_cost: int = 3) -> Schedule:
 
     prio = [0] * n
     for i in range(n - 1, -1, -1):
-        own = recip_cost if ops[i][0] == "D" else 1
+        own = special_cost if ops[i][0] == "D" else 1
         best = own
         for j, k in succ[i]:
             step = 0 if k == "W" else own + (VISIBLE - 1 if k == "R" and ops[i][0] == "F" else 0)
@@ -132,7 +136,7 @@ def schedule(ops, width: int, recip_cost: int = 3) -> Schedule:
     lane_acc = [None] * width            # the operation whose result a lane's accumulator holds
     product = [None] * width             # the MULACC that waits for it
     read = [any(k == "R" for _, k in s) for s in succ]   # others load the result
-    kind = [op[5] for op in ops]
+    kind = [op[5] for op in ops]         # of special operations: not read
     store = [True] * n
     rows, t, done = [], 0, 0
 
@@ -146,17 +150,17 @@ def schedule(ops, width: int, recip_cost: int = 3) -> Schedule:
     ready_at = {i: 0 for i in waiting}
     while done < n:
         ready = [i for i in waiting if ready_at[i] <= t]
-        recips = sorted((i for i in ready if ops[i][0] == "D"), key=lambda i: (-prio[i], i))[:width]
+        specials = sorted((i for i in ready if ops[i][0] == "D"), key=lambda i: (-prio[i], i))[:width]
         # operations that a lane can go on with in its accumulator
         goes_on = {i for i in waiting if chain[i] is not None and ops[i][0] == ops[chain[i]][0] == "F"
                    and lane_acc[lane_of[chain[i]]] == chain[i] and earliest(i, skip_chain=True) <= t}
         cand = sorted(goes_on.union(i for i in ready if ops[i][0] == "F" and ops[i][5] != MULACC),
                       key=lambda i: (-prio[i], i))
-        if recips and t % UNROLL == 0 and (not cand or prio[recips[0]] >= prio[cand[0]] - SLACK):
-            rows.append(("D", recips + [None] * (width - len(recips))))
-            for lane, i in enumerate(recips):
+        if specials and t % UNROLL == 0 and (not cand or prio[specials[0]] >= prio[cand[0]] - SLACK):
+            rows.append(("D", specials + [None] * (width - len(specials))))
+            for lane, i in enumerate(specials):
                 when[i], lane_of[i] = t - 1, lane
-            placed = recips
+            placed = specials
         else:
             lanes, fresh = [None] * width, []
             for i in goes_on:            # a product's accumulator waits for it
@@ -207,15 +211,17 @@ def encode(ops, sch: Schedule, offset, const_offset, zero: int) -> list[list[tup
     for what, lanes in sch.rows:
         row = []
         for i in lanes:
-            if what == "D":
-                row.append((zero | A_RECIP | zero << 16, zero if i is None else offset(ops[i][1]) | D_STORE))
-                continue
             if i is None:
-                row.append(idle)
+                row.append(idle if what == "F" else (zero | A_SPECIAL | zero << 16, zero))
                 continue
-            _, d, a, b, neg, _ = ops[i]
-            k = sch.kind[i]
+            _, d, a, b, neg, special = ops[i]
             const = isinstance(b, tuple)
+            if what == "D":
+                row.append(((zero if a is None else offset(a)) | A_SPECIAL
+                            | (const_offset(b[1]) if const else offset(b)) << 16,
+                            offset(d) | special | D_STORE | (B_CONST if const else 0)))
+                continue
+            k = sch.kind[i]
             w0 = (zero if k == MULACC else offset(a)) | (const_offset(b[1]) if const else offset(b)) << 16
             w1 = (offset(d) | ADDEND[k]) + (D_STORE if sch.store[i] else 0)
             row.append((w0, w1 + (B_CONST if const else 0) + (A_NEG if neg else 0)))
@@ -271,10 +277,10 @@ def tendency(P: Program, m, sp, dst: str):
             P.fma(f"{dst}{s}", f"X{r}", ("c", c), init=NEG0 if t == 0 else LOAD)
 
 
-def partials(P: Program, m, sp):
+def partials(P: Program, m, sp, src: str = "Y"):
     """Partial-derivative products of 2- and 3-reactant reactions (rbjacob.F:112-143)."""
     for r in sp.active[0]:
-        y = [f"Y{sp.irm2[r][q]}" for q in range(m.nreact[r])]
+        y = [f"{src}{sp.irm2[r][q]}" for q in range(m.nreact[r])]
         if m.nreact[r] == 2:
             P.fma(f"E{r}_0", f"R{r}", y[1], init=NEG0)
             P.fma(f"E{r}_1", f"R{r}", y[0], init=NEG0)
@@ -301,23 +307,26 @@ def iteration_matrix(P: Program, m, sp):
             if not tl:
                 empty.add(st)
 
-        def first(st):
-            if st in empty:
-                empty.discard(st)
-                return NEG0
-            return LOAD
         di = jpt[(i, i)]
-        P.fma(f"A{di}", "G", ("c", -1.0), init=first(di))
-        for st, k in sp.lower[0][i]:
-            if st in empty:
-                raise ValueError("an entry of L without terms or updates")
-            P.fma(f"A{st}", f"A{st}", f"A{jpt[(k, k)]}", init=NEG0)
-            for st_kj, j in sp.upper[0][k]:
-                o = jpt[(i, j)]
-                P.fma(f"A{o}", f"A{st}", f"A{st_kj}", neg=True, init=first(o))
-        if empty:
-            raise ValueError("an entry of U without terms or updates")
-        P.recip(f"A{di}")
+        P.fma(f"A{di}", "G", ("c", -1.0), init=NEG0 if di in empty else LOAD)
+        empty.discard(di)
+        eliminate(P, sp, i, empty)
+
+
+def eliminate(P: Program, sp, i: int, empty: set):
+    """Row i's elimination by the rows above; `empty`: its entries without terms, not yet formed."""
+    jpt = sp.jarraypt[0]
+    for st, k in sp.lower[0][i]:
+        if st in empty:
+            raise ValueError("an entry of L without terms or updates")
+        P.fma(f"A{st}", f"A{st}", f"A{jpt[(k, k)]}", init=NEG0)
+        for st_kj, j in sp.upper[0][k]:
+            o = jpt[(i, j)]
+            P.fma(f"A{o}", f"A{st}", f"A{st_kj}", neg=True, init=NEG0 if o in empty else LOAD)
+            empty.discard(o)
+    if empty:
+        raise ValueError("an entry of U without terms or updates")
+    P.special(RCP, f"A{jpt[(i, i)]}", None, f"A{jpt[(i, i)]}")
 
 
 def substitution(P: Program, m, sp, v: str):
@@ -345,6 +354,14 @@ def ros3_programs(m, sp) -> dict[str, Program]:
     tendency(p["rhs"], m, sp, "T")
     substitution(p["solve"], m, sp, "V")
     return p
+
+
+def place(ops, where):
+    """The operations with elements named by their places, so that elements that share a place
+    depend on one another."""
+    def at(e):
+        return e if e is None or isinstance(e, tuple) else where[e]
+    return [(k, at(d), at(a), at(b), neg, init) for k, d, a, b, neg, init in ops]
 
 
 class Ros3Layout:
@@ -384,11 +401,7 @@ class Ros3Layout:
         self.cells = room // (8 * self.elems)
 
     def place(self, ops):
-        """The operations with elements named by their places, so that elements that share a
-        place depend on one another."""
-        def at(e):
-            return e if e is None or isinstance(e, tuple) else self.at[e]
-        return [(k, at(d), at(a), at(b), neg, init) for k, d, a, b, neg, init in ops]
+        return place(ops, self.at)
 
 
 WIDTH = 32           # lanes of a cell (16, two cells to a warp: 8 % slower, the rows are fewer but wait longer)
@@ -408,33 +421,396 @@ def ros3_tables(mech: str, width: int = WIDTH):
     return lay, consts, tables
 
 
+class GearLayout:
+    """Places of SMVGEAR's programs in the one-cell workspace of the Gear kernels (emit_cuda.Layout):
+    a pivot's reciprocal takes the pivot's place, the concentrations with CEFF's zeros the place of
+    VDIAG, and the coefficients times R1DELT that of the rates, which are formed after the
+    matrix, and of the scratch array.  R1DELT, 0 and 1 lie before the workspace."""
+
+    WORKSPACE = 4
+
+    def __init__(self, m, sp, coefs):
+        lay = Layout(m, sp)
+        n, nr, w = m.nspec, m.nrxns, self.WORKSPACE
+        self.q = w + lay.vdiag
+        self.at = dict(H=0, Z=1, O=2)
+        for v, off in (("Y", lay.y), ("U", lay.ydot), ("Q", lay.vdiag)):
+            self.at.update({f"{v}{i}": w + off + i for i in range(n)})
+        for v, off in (("R", lay.rki), ("X", lay.rxrat)):
+            self.at.update({f"{v}{r}": w + off + r for r in range(nr)})
+        self.at.update({f"E{r}_{q}": w + off for (r, q), off in lay.ex.items()})
+        self.at.update({f"A{st}": w + lay.lu + st for st in range(1, sp.iarray[0] + 1)})
+        slots = list(range(lay.rxrat, lay.rxrat + nr)) + list(range(lay.yp, lay.yp + n))
+        if len(coefs) > len(slots):
+            raise ValueError("no room for the scaled coefficients")
+        self.at.update({f"S{q}": w + slots[q] for q in range(len(coefs))})
+        self.elems = w + lay.gear_total
+        if 8 * max(self.at.values()) >= 1 << 16:
+            raise ValueError("an operation's offsets have 16 bits")
+
+
+def gear_programs(m, sp) -> tuple[dict[str, Program], list]:
+    """Of one SMVGEAR evaluation: predictor (P = I - ASN1*DELT*J at the concentrations Q, with R1DELT =
+    -ASN1*DELT in H, and its factors: grpderiv.F:131-226, grdecomp.F), rhs (U = f(Y), grsubfun.F) and
+    solve (U, grbacksub.F).  Returns the programs and the coefficients that are scaled by R1DELT."""
+    terms = _jac_terms(m, sp, 0)
+    coefs = sorted({c for tl in terms.values() for _, _, c, sign in tl if sign > 0 and c is not None})
+    slot = {c: f"S{q}" for q, c in enumerate(coefs)}
+    p = {"predictor": Program(), "rhs": Program(), "solve": Program()}
+    P = p["predictor"]
+    for c in coefs:
+        P.fma(slot[c], "H", ("c", c), init=NEG0)
+    partials(P, m, sp, "Q")
+    jpt = sp.jarraypt[0]
+    for i in range(sp.ischan):
+        di = jpt[(i, i)]
+        empty = set()
+        for st in [st for st, _ in sp.lower[0][i]] + [di] + [st for st, _ in sp.upper[0][i]]:
+            if st == di:
+                P.fma(f"A{st}", "O", ("c", 1.0), init=NEG0)
+            elif not terms.get(st):
+                empty.add(st)
+            for q, (r, ial, coef, sign) in enumerate(terms.get(st, [])):
+                a = f"R{r}" if m.nreact[r] == 1 else f"E{r}_{ial}"
+                P.fma(f"A{st}", a, "H" if sign < 0 or coef is None else slot[coef], neg=sign < 0,
+                      init=NEG0 if q == 0 and st != di else LOAD)
+        eliminate(P, sp, i, empty)
+    rates(p["rhs"], m, sp, "Y")
+    tendency(p["rhs"], m, sp, "U")
+    substitution(p["solve"], m, sp, "U")
+    return p, coefs
+
+
+def gear_tables(mech: str, width: int = WIDTH):
+    """(layout, constants, {program: encoded rows})."""
+    m, sp = mechanism(mech)
+    progs, coefs = gear_programs(m, sp)
+    lay = GearLayout(m, sp, coefs)
+    consts = sorted({op[3][1] for p in progs.values() for op in p.ops if isinstance(op[3], tuple)})
+    cof = {c: 8 * q for q, c in enumerate(consts)}
+    tables = {}
+    for name, p in progs.items():
+        ops = place(p.ops, lay.at)
+        tables[name] = encode(ops, schedule(ops, width), lambda e: 8 * e, lambda c: cof[c], 8 * lay.at["Z"])
+    return lay, consts, tables
+
+
+# ----------------------------------------------------------------------------- EBI
+# HRRATES, HRG1-HRG4 and HRPRODLOSS as straight-line C (gen/<mech>_ebi.cu), turned into operations.
+# Their products and sums are rounded one by one (no fused multiply-add in the EBI code), so a term
+# takes a product and an addition, x * 1.0 + acc, unless its factor is a power of two: such a
+# product is exact, and the fused operation gives the same sum.
+
+_TOKEN = re.compile(r"\s*(?:(\d+\.?\d*(?:e[-+]?\d+)?)|(EBI_\w+)\((\d+)\)|(\w+)|(.))")
+_EBI_ARRAYS = {"EBI_YC": "C", "EBI_YC0": "B", "EBI_YCP": "P", "EBI_RKI": "R", "EBI_RXRAT": "X", "EBI_PROD": "M",
+               "EBI_LOSS": "L", "EBI_PNEG": "N"}
+
+
+def _parse(text: str):
+    """An expression of numbers, elements, + - * /, fmax, sqrt, fabs and copysign as nested tuples."""
+    toks = []
+    for num, arr, idx, name, ch in _TOKEN.findall(text):
+        toks.append(("num", float(num)) if num else ("el", _EBI_ARRAYS[arr] + idx) if arr else
+                    ("name", name) if name else (ch, None))
+    pos = 0
+
+    def peek():
+        return toks[pos][0] if pos < len(toks) else None
+
+    def take(kind=None):
+        nonlocal pos
+        t = toks[pos]
+        if kind is not None and t[0] != kind:
+            raise ValueError(f"expected {kind} in {text}")
+        pos += 1
+        return t
+
+    def atom():
+        t = take()
+        if t[0] in ("num", "el"):
+            return t
+        if t[0] == "-":
+            e = atom()
+            return ("num", -e[1]) if e[0] == "num" else ("neg", e)
+        if t[0] == "(":
+            e = add()
+            take(")")
+            return e
+        if t[0] == "name" and peek() == "(":
+            take("(")
+            args = [add()]
+            while peek() == ",":
+                take(",")
+                args.append(add())
+            take(")")
+            return (t[1], *args)
+        if t[0] == "name":
+            return ("el", t[1])
+        raise ValueError(f"unexpected {t} in {text}")
+
+    def mul():
+        e = atom()
+        while peek() in ("*", "/"):
+            op = take()[0]
+            e = (op, e, atom())
+        return e
+
+    def add():
+        e = mul()
+        while peek() in ("+", "-"):
+            op = take()[0]
+            e = (op, e, mul())
+        return e
+
+    e = add()
+    if pos != len(toks):
+        raise ValueError(f"trailing text in {text}")
+    return e
+
+
+class _Emit:
+    """Expressions to operations; temporaries come from a ring of places."""
+
+    def __init__(self, P: Program, temps: int):
+        self.P, self.temps, self.next = P, temps, 0
+
+    def temp(self):
+        self.next += 1
+        return f"t{(self.next - 1) % self.temps}"
+
+    @staticmethod
+    def exact(v: float) -> bool:
+        return v != 0.0 and abs(math.frexp(v)[0]) == 0.5
+
+    def operand(self, e):
+        """An element that holds the value of e (constants have no element: see `b`)."""
+        return e[1] if e[0] == "el" else self.value(e)
+
+    def value(self, e, dst=None):
+        """e's value in dst or a new temporary; returns the element."""
+        P, kind = self.P, e[0]
+        if kind == "el":
+            if dst is None:
+                return e[1]
+            P.fma(dst, e[1], ("c", 1.0), init=NEG0)
+            return dst
+        if kind == "num":
+            dst = dst or self.temp()
+            P.fma(dst, "O", ("c", e[1]), init=NEG0)
+            return dst
+        if kind == "neg":
+            a = self.operand(e[1])
+            dst = dst or self.temp()
+            P.fma(dst, a, ("c", 1.0), neg=True, init=NEG0)
+            return dst
+        if kind == "*":
+            x, y = e[1], e[2]
+            if x[0] == "num":
+                x, y = y, x
+            if x[0] == "num":
+                raise ValueError("a product of constants")
+            if x[0] != "el" and y[0] != "num" and y[0] == "el":
+                pass
+            a = self.operand(x)
+            b = ("c", y[1]) if y[0] == "num" else self.operand(y)
+            dst = dst or self.temp()
+            P.fma(dst, a, b, init=NEG0)
+            return dst
+        if kind in "+-":
+            terms = []                       # a left-associated sum: its terms in order
+            while e[0] in ("+", "-"):
+                terms.append((e[0], e[2]))
+                e = e[1]
+            acc = self.temp()                # not dst itself, which a later term may read
+            if e[0] == "num" and e[1] == 1.0:
+                P.fma(acc, "O", ("c", 1.0), init=NEG0)
+            else:
+                self.value(e, acc)
+            for sign, t in reversed(terms):
+                neg = sign == "-"
+                if t[0] == "*" and t[1][0] == "num" and self.exact(t[1][1]):
+                    P.fma(acc, self.operand(t[2]), ("c", t[1][1]), neg=neg)
+                elif t[0] == "num":
+                    P.fma(acc, "O", ("c", t[1]), neg=neg)
+                else:
+                    P.fma(acc, self.operand(t), ("c", 1.0), neg=neg)
+            if dst is None:
+                return acc
+            P.fma(dst, acc, ("c", 1.0), init=NEG0)
+            return dst
+        if kind == "/":
+            b = self.operand(e[2])
+            if e[1] == ("num", 1.0):
+                dst = dst or self.temp()
+                P.special(RCP, dst, None, b)
+                return dst
+            a = self.operand(e[1])
+            dst = dst or self.temp()
+            P.special(DIV, dst, a, b)
+            return dst
+        if kind == "fmax":
+            a = "Z" if e[1] == ("num", 0.0) else self.operand(e[1])
+            b = self.operand(e[2])
+            dst = dst or self.temp()
+            P.special(MAX, dst, a, b)
+            return dst
+        if kind == "sqrt":
+            b = self.operand(e[1])
+            dst = dst or self.temp()
+            P.special(SQRT, dst, None, b)
+            return dst
+        if kind == "copysign" and e[1] == ("fabs", ("num", 1.0)):
+            b = self.operand(e[2])
+            dst = dst or self.temp()
+            P.special(SIGN, dst, None, b)
+            return dst
+        raise ValueError(f"unknown expression {kind}")
+
+
+def ebi_program(mech: str, temps: int = 768) -> Program:
+    """One iteration's HRRATES, HRG1-HRG4 and HRPRODLOSS."""
+    text = (PKG / "csrc" / "gen" / f"{mech}_ebi.cu").read_text()
+    P = Program()
+    em = _Emit(P, temps)
+    for name in ("hrrates", "hrg1", "hrg2", "hrg3", "hrg4", "hrprodloss"):
+        body = re.search(rf"void ebi_{name}\([^)]*\)\n\{{\n(.*?)\n\}}", text, re.S).group(1)
+        own = {}
+        for line in body.splitlines():
+            line = line.strip()
+            if line.startswith(("double ", "(void)")):
+                continue
+            lhs, rhs = line.rstrip(";").split(" = ", 1)
+            e = _parse(rhs)
+            d = _parse(lhs)[1]
+
+            def local(x):          # a routine's own variables: each assignment is a new element
+                if x[0] == "el":
+                    return ("el", own.get(x[1], x[1]))
+                return tuple(local(y) if isinstance(y, tuple) else y for y in x)
+            e = local(e)
+            if d.startswith("l_") or d == "dtc":
+                own[d] = e[1] if e[0] == "el" else em_keep(em, e)
+            elif e[0] == "num":
+                P.fma(d, "Z" if e[1] == 0.0 else "O", ("c", 1.0 if e[1] == 0.0 else e[1]), init=NEG0)
+            elif name == "hrrates":
+                rate_chain(P, em, d, e)
+            else:
+                em.value(e, d)
+    return P
+
+
+def em_keep(em, e):
+    """e's value in an element of its own (a routine's variable lives longer than a temporary)."""
+    em.kept = getattr(em, "kept", 0) + 1
+    return em.value(e, f"v{em.kept - 1}")
+
+
+def rate_chain(P, em, d, e):
+    """RKI * YC * YC ...: the products in place."""
+    if e[0] == "el":
+        P.fma(d, e[1], ("c", 1.0), init=NEG0)
+        return
+    if e[0] != "*":
+        raise ValueError("a rate is a product")
+    if e[1][0] == "el":
+        P.fma(d, e[1][1], e[2][1], init=NEG0)
+        return
+    rate_chain(P, em, d, e[1])
+    P.fma(d, None, e[2][1], init=MULACC)
+
+
+class EbiLayout:
+    """Element offsets (doubles) of a cell's EBI state in shared memory."""
+
+    def __init__(self, m, P: Program):
+        n, nr = m.nspec, m.nrxns
+        self.at, off = {}, 0
+        for v in "CBPMLN":                    # YC, YC0, YCP, PROD, LOSS, PNEG
+            self.at.update({f"{v}{i}": off + i for i in range(n)})
+            setattr(self, "yc yc0 ycp prod loss pneg".split()["CBPMLN".index(v)], off)
+            off += n
+        for v, name in (("R", "rki"), ("X", "rxrat")):
+            self.at.update({f"{v}{r}": off + r for r in range(nr)})
+            setattr(self, name, off)
+            off += nr
+        self.dtc, self.z, self.one = off, off + 1, off + 2
+        self.at.update(dtc=off, Z=off + 1, O=off + 2)
+        off += 3
+        used = {x for op in P.ops for x in (op[1], op[2], op[3]) if isinstance(x, str)}
+        for e in sorted(used - set(self.at), key=lambda x: (x[0], int(x[1:]))):
+            self.at[e] = off
+            off += 1
+        self.elems = off
+
+
+def ebi_tables(mech: str, width: int = WIDTH):
+    """(layout, constants, encoded rows)."""
+    m, _ = mechanism(mech)
+    P = ebi_program(mech)
+    lay = EbiLayout(m, P)
+    consts = sorted({op[3][1] for op in P.ops if isinstance(op[3], tuple)})
+    cof = {c: 8 * q for q, c in enumerate(consts)}
+    ops = place(P.ops, lay.at)
+    return lay, consts, encode(ops, schedule(ops, width), lambda e: 8 * e, lambda c: cof[c], 8 * lay.z)
+
+
+def _rows_text(sym, tables, chunk):
+    """Programs one after the other, each from the start of a chunk: (declaration, definition)."""
+    rows = []
+    for table in tables:
+        rows += table
+        rows += [[(0, 0)] * WIDTH] * (-len(rows) % chunk)
+    size = len(rows) * WIDTH
+    return (f"extern __device__ const uint2 {sym}[{size}];",
+            [f"__device__ __align__(128) const uint2 {sym}[{size}] = {{"]
+            + ["  " + ", ".join(f"{{0x{a:x}u, 0x{b:x}u}}" for a, b in row) + "," for row in rows] + ["};"])
+
+
+def _consts_text(sym, consts):
+    return (f"extern __device__ const double {sym}[{len(consts)}];",
+            f"__device__ const double {sym}[{len(consts)}] = {{{', '.join(map(c_double, consts))}}};")
+
+
 def sources(mech: str) -> dict[str, str]:
     """<mech>_coop.cuh (sizes) and <mech>_coop.cu (tables)."""
-    lay, consts, tables = ros3_tables(mech)
-    banner = [f"// Generated by cmaq_gb300.mechgen.coop from mechs/{mech}/manifest.json.  Do not edit."]
+    banner = [f"// Generated by cmaq_gb300.mechgen.coop from mechs/{mech}/manifest.json and gen/{mech}_ebi.cu.  Do not edit."]
     ns = f"mech_{mech}"
-    h = banner + ["// Sizes and tables of the cooperative ROS3 kernel (csrc/coop.cuh).", "#pragma once",
-                  "#include <cuda_runtime.h>", f"namespace {ns} {{",
-                  f"extern __device__ const double c_coop_const[{len(consts)}];"]
-    c = banner + [f'#include "{mech}_coop.cuh"', f"namespace {ns} {{",
-                  f"__device__ const double c_coop_const[{len(consts)}] = {{{', '.join(map(c_double, consts))}}};"]
-    rows = []                # programs one after the other, each from the start of a chunk
-    for table in tables.values():
-        rows += table
-        rows += [[(0, 0)] * WIDTH] * (-len(rows) % CHUNK)
-    h.append(f"extern __device__ const uint2 c_coop_rows[{len(rows) * WIDTH}];")
-    c.append(f"__device__ __align__(128) const uint2 c_coop_rows[{len(rows) * WIDTH}] = {{")
-    c += ["  " + ", ".join(f"{{0x{a:x}u, 0x{b:x}u}}" for a, b in row) + "," for row in rows]
-    c.append("};")
-    h += ["struct Coop {",
-          f"    static constexpr int ELEMS = {lay.elems}, NCONST = {len(consts)}, MAX_CELLS = {lay.cells};",
-          f"    static constexpr int Y = {lay.y}, V = {lay.v}, K1 = {lay.k}, K2 = {lay.l}, T = {lay.t};",
-          f"    static constexpr int RKI = {lay.rki}, G = {lay.g}, Z = {lay.z};",
-          f"    static constexpr int CHUNK = {CHUNK}, TABLE_SMEM = {TABLE_SMEM};",
-          "    static __device__ __forceinline__ const double* constants() { return c_coop_const; }",
-          "    static __device__ __forceinline__ const uint2* rows() { return c_coop_rows; }",
-          "    static constexpr int " + ", ".join(f"{n.upper()}_ROWS = {len(t)}" for n, t in tables.items()) + ";"]
-    h += ["};", f"}}  // namespace {ns}"]
+    h = banner + ["// Sizes and tables of the cooperative kernels (csrc/coop.cuh, csrc/ebi_coop.cuh).", "#pragma once",
+                  "#include <cuda_runtime.h>", f"namespace {ns} {{"]
+    c = banner + [f'#include "{mech}_coop.cuh"', f"namespace {ns} {{"]
+
+    def traits(name, lay, consts, progs, fields, seq, at, chunk=CHUNK):
+        low = name.lower()
+        for d, t in (_consts_text(f"c_{low}_const", consts), _rows_text(f"c_{low}_rows", progs.values(), chunk)):
+            h.append(d)
+            c.extend(t if isinstance(t, list) else [t])
+        n = {k: -(-len(t) // chunk) for k, t in progs.items()}
+        table = 2 * (chunk + AHEAD) * WIDTH * 8 + 64
+        cells = (SMEM_MAX - table - 8 * len(consts)) // (8 * lay.elems)
+        return [f"struct {name} {{",
+                f"    static constexpr int ELEMS = {lay.elems}, NCONST = {len(consts)}, MAX_CELLS = {cells};",
+                "    static constexpr int " + ", ".join(f"{k} = {v}" for k, v in fields.items()) + ";",
+                f"    static constexpr int CHUNK = {chunk}, TABLE_SMEM = {table};",
+                "    static constexpr int " + ", ".join(f"{k.upper()}_ROWS = {len(t)}" for k, t in progs.items()) + ";",
+                f"    // chunks of one pass through the programs ({', '.join(seq)}), and where each lies",
+                f"    static constexpr int PASS = {sum(n[k] for k in seq)};",
+                f"    static __device__ __forceinline__ int chunk(int k) {{ return {at(n)}; }}",
+                f"    static __device__ __forceinline__ const double* constants() {{ return c_{low}_const; }}",
+                f"    static __device__ __forceinline__ const uint2* rows() {{ return c_{low}_rows; }}", "};"]
+    lay, consts, tables = ros3_tables(mech)
+    tail = traits("Coop", lay, consts, tables,
+                  dict(Y=lay.y, V=lay.v, K1=lay.k, K2=lay.l, T=lay.t, RKI=lay.rki, G=lay.g, Z=lay.z),
+                  ["stage1", "rhs", "solve", "solve"],
+                  lambda n: f"k < {sum(n.values())} ? k : k - {n['solve']}")
+    elay, econsts, rows = ebi_tables(mech)
+    tail += traits("CoopEbi", elay, econsts, {"iteration": rows},
+                   dict(YC=elay.yc, YC0=elay.yc0, YCP=elay.ycp, PROD=elay.prod, LOSS=elay.loss, PNEG=elay.pneg,
+                        RKI=elay.rki, DTC=elay.dtc, Z=elay.z, ONE=elay.one), ["iteration"], lambda n: "k")
+    glay, gconsts, gtabs = gear_tables(mech)
+    # one-warp blocks with a stream each: chunks as large as leave room for 4 (CB6r5) and 3 (CRACMM2) on an SM
+    tail += traits("CoopGear", glay, gconsts, gtabs, dict(Q=glay.q, R1=0, Z=1, ONE=2, WORKSPACE=glay.WORKSPACE),
+                   ["predictor", "rhs", "solve"], lambda n: "k", 16 if glay.elems < 6000 else 8)
+    h += tail + [f"}}  // namespace {ns}"]
     c.append(f"}}  // namespace {ns}")
     return {f"{mech}_coop.cuh": "\n".join(h) + "\n", f"{mech}_coop.cu": "\n".join(c) + "\n"}
 

@@ -230,11 +230,7 @@ def cuda_sources(m: Mechanism, prog: RateProgram, sp: SparseMech, mech: str, src
               ("GEAR_WS_ELEMS", lay.gear_total), ("GEAR_CNEW", lay.y), ("GEAR_GLOSS", lay.ydot),
               ("GEAR_DTLOS", lay.k1), ("GEAR_CHOLD", lay.k2), ("GEAR_CEST", lay.k3), ("GEAR_BLKCONC", lay.f0),
               ("GEAR_CONC", lay.gear_conc), ("GEAR_E", lay.yp), ("GEAR_CAVEG", lay.yave),
-              ("GEAR_CFINI", lay.gear_cfini),
-              # warp-cooperative EBI: one cell's state in shared memory (doubles)
-              ("EBIW_YC", 0), ("EBIW_YC0", ns), ("EBIW_YCP", 2 * ns), ("EBIW_PROD", 3 * ns),
-              ("EBIW_LOSS", 4 * ns), ("EBIW_PNEG", 5 * ns), ("EBIW_NOTMAX", 6 * ns), ("EBIW_RKI", 7 * ns),
-              ("EBIW_RXRAT", 7 * ns + nr), ("EBIW_ELEMS", 7 * ns + 2 * nr))
+              ("GEAR_CFINI", lay.gear_cfini))
     for k, v in consts:
         h.append(f"constexpr int {k} = {v};")
     h.append(f"constexpr double FLOPS_STEP_DAY = {float(flop_counts(m, sp, 0)['step_total'])};")
@@ -284,17 +280,6 @@ def cuda_sources(m: Mechanism, prog: RateProgram, sp: SparseMech, mech: str, src
             h.append(f"    static __device__ __forceinline__ void ebi_{nm}(double* ws) {{ {ns_name}::ebi_{nm}(ws); }}")
         for nm in ("hrg1", "hrg2", "hrg3", "hrg4"):
             h.append(f"    static __device__ __forceinline__ void ebi_{nm}(double* ws, double dtc) {{ {ns_name}::ebi_{nm}(ws, dtc); }}")
-            h.append(f"    static __device__ __forceinline__ void ebiw_{nm}(double* sm, double dtc) {{ {ns_name}::wsm::ebi_{nm}(sm, dtc); }}")
-        h.append(f"    static constexpr int EBIW_NRATE = {ns_name}::EBIW_NRATE;")
-        h.append(f"    static __device__ __forceinline__ const int* ebiw_rate_r() {{ return {ns_name}::c_ebiw_rate_r; }}")
-        h.append(f"    static __device__ __forceinline__ const int* ebiw_rate_nf() {{ return {ns_name}::c_ebiw_rate_nf; }}")
-        h.append(f"    static __device__ __forceinline__ const int* ebiw_rate_sp() {{ return {ns_name}::c_ebiw_rate_sp; }}")
-        h.append(f"    static __device__ __forceinline__ const int* ebiw_pl_ptr() {{ return {ns_name}::c_ebiw_pl_ptr; }}")
-        h.append(f"    static __device__ __forceinline__ const int* ebiw_pl_kind() {{ return {ns_name}::c_ebiw_pl_kind; }}")
-        h.append(f"    static __device__ __forceinline__ const int* ebiw_pl_sp() {{ return {ns_name}::c_ebiw_pl_sp; }}")
-        h.append(f"    static __device__ __forceinline__ const int* ebiw_pl_t0() {{ return {ns_name}::c_ebiw_pl_t0; }}")
-        h.append(f"    static __device__ __forceinline__ const int* ebiw_term_r() {{ return {ns_name}::c_ebiw_term_r; }}")
-        h.append(f"    static __device__ __forceinline__ const double* ebiw_term_c() {{ return {ns_name}::c_ebiw_term_c; }}")
     for k, v in gw_info["sizes"].items():
         h.append(f"    static constexpr int {k} = {v};")
     for k in gw_info["names"]:

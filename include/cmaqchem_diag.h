@@ -61,7 +61,7 @@ int cmaqchem_diag_fp64_issue(int device, int active_lanes, double* cycles_per_in
  * "ebi_warp" (EBI solver: 1 (default) one cell per warp with its state in shared memory,
  * 0 one cell per lane; same results), "ebi_defer" (EBI: n > 0 runs one cell per lane and
  * hands the cells still iterating after n Backward-Euler iterations to the one-cell-per-warp
- * kernel, which integrates them from their inputs; default 100; 0: ebi_warp alone decides;
+ * kernel, which integrates them from their inputs; 0 (default): ebi_warp alone decides;
  * same results) and
  * "gear_warp" (SMVGEAR: 1 (default) one cell per warp with its workspace in shared memory,
  * 0 one cell per lane; same results). */

@@ -21,10 +21,10 @@ class Terms:
 def sequential(ops, start, term):
     x = dict(start)
     for kind, d, a, b, neg, init in ops:
-        if kind == "D":
-            x[d] = term("rcp", x[d])
-            continue
         vb = term("const", b[1]) if isinstance(b, tuple) else x[b]
+        if kind == "D":
+            x[d] = term("special", init, x[a] if init in (C.DIV, C.MAX) else None, vb)
+            continue
         va = x[d] if init == C.MULACC else x[a]
         x[d] = term("fma", neg, va, vb, x[d] if init == C.LOAD else "-0")
     return x
@@ -45,21 +45,22 @@ def rows_run(rows, start, consts, term):
 
     idle = [(0, 0)] * width
     at = lambda t: load(rows[t] if t < len(rows) else idle)
-    ops, pending, recip = [at(0), at(1)], {}, False
+    ops, pending, special = [at(0), at(1)], {}, False
     for t, row in enumerate(rows):
         if t % C.UNROLL == 0:
-            recip = bool(row[0][0] & C.A_RECIP)
-            if recip:                                      # a block of its own: the rest of it is not read
+            special = bool(row[0][0] & C.A_SPECIAL)
+            if special:                                      # a block of its own: the rest of it is not read
                 x.update(pending)
                 pending = {}
-                assert all(w0 & C.A_RECIP for w0, _ in row)
-                for w0, w1 in row:
-                    if w1 & C.D_STORE:
-                        x[(w1 & 0xfff8) // 8] = term("rcp", x[(w1 & 0xfff8) // 8])
+                assert all(w0 & C.A_SPECIAL for w0, _ in row)
+                got = [(w1, v) for (_, w1), v in zip(row, load(row)) if w1 & C.D_STORE]
+                for w1, (a, b, _) in got:
+                    kind = w1 & 7
+                    x[(w1 & 0xfff8) // 8] = term("special", kind, a if kind in (C.DIV, C.MAX) else None, b)
                 ops = [at(t + C.UNROLL), at(t + C.UNROLL + 1)]
-        if recip:
+        if special:
             continue
-        assert not any(w0 & C.A_RECIP for w0, _ in row)
+        assert not any(w0 & C.A_SPECIAL for w0, _ in row)
         cur, results = ops.pop(0), {}
         for ln, (w0, w1) in enumerate(row):
             a, b, c = cur[ln]
@@ -94,6 +95,32 @@ def test_rows_carry_out_the_sequential_operations(mech, width):
         got = rows_run(tables[name], start, consts, term)
         # partial-derivative products are scratch: elements that nothing reads any more
         scratch = set(lay.alias.values()) if name == "stage1" else set()
+        assert all(got[e] == want[e] for e in range(lay.elems) if e not in scratch), name
+
+
+@pytest.mark.parametrize("mech", ["cb6r5_ae7_aq", "cracmm2"])
+@pytest.mark.parametrize("width", [C.WIDTH, 8])
+def test_ebi_rows_carry_out_the_sequential_operations(mech, width):
+    lay, consts, rows = C.ebi_tables(mech, width)
+    ops = C.place(C.ebi_program(mech).ops, lay.at)
+    term = Terms()
+    start = {e: term("in", e) for e in range(lay.elems)}
+    want, got = sequential(ops, start, term), rows_run(rows, start, consts, term)
+    assert all(got[i] == want[i] for i in range(lay.elems)
+               if i in {lay.at[e] for e in lay.at if e[0] in "CBPMLNRX"})
+
+
+@pytest.mark.parametrize("mech", ["cb6r5_ae7_aq", "cracmm2"])
+def test_gear_rows_carry_out_the_sequential_operations(mech):
+    m, sp = C.mechanism(mech)
+    lay, consts, tables = C.gear_tables(mech)
+    progs, coefs = C.gear_programs(m, sp)
+    for name, prog in progs.items():
+        ops = C.place(prog.ops, lay.at)
+        term = Terms()
+        start = {e: term("in", e) for e in range(lay.elems)}
+        want, got = sequential(ops, start, term), rows_run(tables[name], start, consts, term)
+        scratch = {lay.at[f"S{q}"] for q in range(len(coefs))} if name == "predictor" else set()
         assert all(got[e] == want[e] for e in range(lay.elems) if e not in scratch), name
 
 

@@ -74,3 +74,22 @@ def test_graph_replay_and_ddm():
         s.step_ddm(sen, conc, *t[1:], rate_mask=mask)
         out.append((conc.cpu().numpy(), sen.cpu().numpy()))
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("mech,dims", [("cb6r5_ae7_aq", (1, 1, 1)), ("cb6r5_ae7_aq", (153, 4, 1)),
+                                       ("cracmm2", (7, 5, 1))])
+def test_ebi_same_bits_as_one_cell_per_lane(mech, dims):
+    _, t, s = setup(mech, dims, seed=35, solver="ebi")
+    s.set_tuning(ebi_warp=1, ebi_defer=0)
+    a = run(s, t, -1)
+    s.set_tuning(ebi_warp=0)
+    same(run(s, t, -1), a)
+
+
+def test_ebi_cells_that_reach_the_iteration_cap():
+    _, t, s = setup("cb6r5_ae7_aq", (13, 5, 2), seed=36, solver="ebi", max_iter=60)
+    s.set_tuning(ebi_warp=1, ebi_defer=0)
+    a = run(s, t, -1, 1)
+    s.set_tuning(ebi_warp=0)
+    assert 0 < a[1][0]["failed_cells"] < 130
+    same(run(s, t, -1, 1), a)
