@@ -399,7 +399,7 @@ extern "C" int cmaqchem_init(const cmaqchem_cfg* cfg, cmaqchem_handle** out)
         CK(cudaMalloc(&h->d_hist, sizeof(unsigned int) * chem::QUEUE_BINS));
         CK(cudaMalloc(&h->d_cursor, sizeof(unsigned long long) * chem::QUEUE_BINS));
         CK(cudaMalloc(&h->d_head, sizeof(unsigned long long)));
-        if (cfg->solver == CMAQCHEM_SOLVER_EBI ||
+        if (cfg->solver == CMAQCHEM_SOLVER_EBI || cfg->solver == CMAQCHEM_SOLVER_GEAR ||
             (cfg->solver == CMAQCHEM_SOLVER_ROS3 &&
              (cfg->schedule == CMAQCHEM_SCHED_QUEUE || use_coop(h, h->ncell)))) {
             // the rate-constant pass's arrays, when they leave a quarter of the free memory
@@ -552,8 +552,17 @@ static int enqueue_step(cmaqchem_handle* h, const chem::GridArgs& a, int itmstep
         if (gear_solver) {
             chem::GearArgs g{};
             g.coef = h->d_gear_coef;
-            if (h->gear_warp) CK(h->ops->gear_warp(a, q, g, true, h->gearw_nblocks, s));
-            else CK(h->ops->gear(a, q, g, true, h->gear_nblocks, s));
+            if (h->gear_warp) {
+                chem::GridArgs ap = a;
+                if (h->d_rki_all) {
+                    CK(h->ops->rconst_pass(a, c0, c1, h->d_rki_all, h->d_sun_all, h->nblocks, s));
+                    ap.rki_all = h->d_rki_all;
+                    ap.sun_all = h->d_sun_all;
+                }
+                CK(h->ops->gear_warp(ap, q, g, true, h->gearw_nblocks, s));
+            } else {
+                CK(h->ops->gear(a, q, g, true, h->gear_nblocks, s));
+            }
         } else if (ebi_solver) {
             chem::EbiArgs e{};
             ebi::steps_for(itmstep, h->ops->ebi_deltat, &e.n_ebi_steps, &e.tmstep);

@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <math_constants.h>
+#include "fpdiv.cuh"
 // GEAR_CELL_ONLY: the per-cell SMVGEAR code without the kernels at the end (the host
 // build of the CPU tests)
 #ifndef GEAR_CELL_ONLY
@@ -177,14 +178,16 @@ static __device__ double gpow(double x, double y)
 
 // The state machine below runs in two forms.  S = 32, COOP = false: one cell per lane on
 // the per-warp workspace ([element][lane]), calling the generated routines.  S = 1,
-// COOP = true: one cell per warp on the warp's shared-memory copy of the cell's workspace;
-// element-wise species loops are spread over the lanes (LOOP, then SYNC) and the f
-// evaluation, P and its LU and the solves run in table-driven cooperative forms
-// (coop_feval, coop_pdecomp, coop_solve), while every lane runs the control flow and the
-// reductions (in the reference's order) itself, so all lanes hold the same state.  Both
-// forms perform the same operations in the same order on every element.
+// COOP = true: one cell per warp on the warp's shared-memory copy of the cell's workspace
+// (gear_coop.cuh); element-wise species loops are spread over the lanes (LOOP, then SYNC),
+// while every lane runs the control flow and the reductions (in the reference's order)
+// itself, so all lanes hold the same state.  Both forms perform the same operations in the
+// same order on every element.  All lanes go through the same trips of a LOOP: lanes that
+// left one early would go through what follows apart from the others.
 #define GW(off) ws[(off) * S]
-#define LOOP(i, n) for (int i = (COOP ? (int)(threadIdx.x & 31) : 0); i < (n); i += (COOP ? 32 : 1))
+#define LOOP(i, n)                                                                                              \
+    for (int b_ = 0, i = (COOP ? (int)(threadIdx.x & 31) : 0); b_ < (n); b_ += (COOP ? 32 : 1), i += (COOP ? 32 : 1)) \
+        if (!COOP || i < (n))
 #define SYNC()                 \
     do {                       \
         if (COOP) __syncwarp(); \
@@ -342,7 +345,7 @@ init_post:
     {
         const double yloweps = s.ylowa / epslow;
         double dely;
-        REDUCE_SQ(dely, GL(j) / (CN(j) + yloweps));
+        REDUCE_SQ(dely, fpdiv::div(GL(j), CN(j) + yloweps));
         const double rmstop = dely > 0.0 ? dely : 0.0;
         double delt = sqrt(epslow / (abst2 + rmstop / order)) * h0fac;
         delt = min2(delt, chemstep);
@@ -406,7 +409,7 @@ loop_order:
         s.rdelmax = 10.0;
         if (s.st.nsteps % 3 == 2) s.ylowa = optimal_atol<M, S>(ws, K);
         const double yloweps1 = s.ylowa * eps1;
-        LOOP(j, isc) CH(j) = eps1 / (fabs(CN(j)) + yloweps1);
+        LOOP(j, isc) CH(j) = fpdiv::div(eps1, fabs(CN(j)) + yloweps1);
         SYNC();
     }
     if (fabs(s.hratio - 1.0) > HRMAX || s.st.nsteps >= s.nslp) s.jeval = 1;
@@ -605,185 +608,45 @@ converged:
 #undef ASET
 }
 
-// ---- warp-cooperative forms of the generated routines (one cell per warp, workspace in
-// shared memory with stride 1), driven by the generator's gw tables.  Each element gets
-// the same operations in the same order as in the generated sequential code.
-
-// GLOSS = f(CNEW): rates over the lanes, then each species' terms in RBFEVAL's order by
-// the lane the species is assigned to
-template <class M>
-__device__ void coop_feval(double* __restrict__ ws)
+// SUBFUN's floor (grsubfun.F:164-171)
+template <class M, int S, bool COOP>
+__device__ __forceinline__ void floor_gloss(double* __restrict__ ws)
 {
-    const int lane = threadIdx.x & 31;
-    const int* ar = M::gw_act_r();
-    const int* asp = M::gw_act_sp();
-    for (int t = lane; t < M::GW_NACT; t += 32) {
-        double x = ws[M::OFF_RKI + ar[t]];
-        const int s0 = asp[3 * t], s1 = asp[3 * t + 1], s2 = asp[3 * t + 2];
-        if (s0 >= 0) x = x * ws[M::GEAR_CNEW + s0];
-        if (s1 >= 0) x = x * ws[M::GEAR_CNEW + s1];
-        if (s2 >= 0) x = x * ws[M::GEAR_CNEW + s2];
-        ws[M::OFF_RXRAT + ar[t]] = x;
+    LOOP(i, M::ISCHAN) {
+        double& g = GW(M::GEAR_GLOSS + i);
+        if (GW(M::GEAR_CNEW + i) <= ZBOUND && g < 0.0) g = 0.0;
     }
-    __syncwarp();
-    const int* lp = M::gw_lane_ptr();
-    const int* ls = M::gw_lane_sp();
-    const int* sptr = M::gw_sum_ptr();
-    const int* sr = M::gw_sum_r();
-    const int* sk = M::gw_sum_k();
-    const double* sc = M::gw_sum_c();
-    for (int u = lp[lane]; u < lp[lane + 1]; ++u) {
-        const int sp = ls[u];
-        const int t0 = sptr[sp], t1 = sptr[sp + 1];
-        double a = 0.0;
-        if (t0 < t1) {
-            const double r0 = ws[M::OFF_RXRAT + sr[t0]];
-            a = sk[t0] ? sc[t0] * r0 : -r0;
-            for (int t = t0 + 1; t < t1; ++t) {
-                const double rr = ws[M::OFF_RXRAT + sr[t]];
-                a = sk[t] ? fma(sc[t], rr, a) : a - rr;
-            }
-        }
-        ws[M::GEAR_GLOSS + sp] = a;
-    }
-    __syncwarp();
+    SYNC();
 }
 
-// P = I - ASN1*DELT*J at CNEW and its LU factors: EXPLIC and the assembly over the lanes,
-// then the elimination pivot by pivot (L entries of the pivot's column scaled, then its
-// updates, each over the lanes)
-template <class M>
-__device__ void coop_pdecomp(double* __restrict__ ws, double r1delt)
+// right-hand side of the corrector's solve (grsmvgear.F:616-620)
+template <class M, int S, bool COOP>
+__device__ __forceinline__ void corrector_rhs(double* __restrict__ ws, double delt)
 {
-    const int lane = threadIdx.x & 31;
-    const int* xr = M::gw_ex_r();
-    const int* xs = M::gw_ex_sp();
-    const int* xo = M::gw_ex_off();
-#define CEFF_(v) ((v) <= 1.0e-30 ? 0.0 : (v))
-    for (int t = lane; t < M::GW_NEX; t += 32) {
-        const double kk = ws[M::OFF_RKI + xr[t]];
-        const double y1 = CEFF_(ws[M::GEAR_CNEW + xs[3 * t]]);
-        const double y2 = CEFF_(ws[M::GEAR_CNEW + xs[3 * t + 1]]);
-        const int o = xo[t];
-        if (xs[3 * t + 2] < 0) {
-            ws[o] = kk * y2;
-            ws[o + 1] = kk * y1;
-        } else {
-            const double y3 = CEFF_(ws[M::GEAR_CNEW + xs[3 * t + 2]]);
-            const double cr2 = kk * y2;
-            ws[o] = cr2 * y3;
-            ws[o + 1] = (kk * y1) * y3;
-            ws[o + 2] = cr2 * y1;
-        }
+    LOOP(i, M::ISCHAN) {
+        double& g = GW(M::GEAR_GLOSS + i);
+        g = fma(delt, g, -(GW(M::GEAR_CONC + M::ISCHAN + i) + GW(M::GEAR_DTLOS + i)));
     }
-#undef CEFF_
-    __syncwarp();
-    double* __restrict__ lu = ws + M::OFF_LU;
-    double* __restrict__ vd = ws + M::OFF_VDIAG;
-    const int* ap = M::gw_asm_ptr();
-    const int* asrc = M::gw_asm_src();
-    const int* ak = M::gw_asm_kind();
-    const double* ac = M::gw_asm_c();
-    constexpr int NST = M::IARRAY_DAY;
-    for (int st = lane + 1; st <= NST; st += 32) {
-        double a = st > NST - M::ISCHAN ? 1.0 : 0.0;   // the diagonal is stored last
-        for (int t = ap[st]; t < ap[st + 1]; ++t) {
-            const double ex = ws[asrc[t]];
-            const int k = ak[t];
-            a = k < 0 ? fma(-r1delt, ex, a) : (k == 0 ? fma(r1delt, ex, a) : fma(ac[t] * r1delt, ex, a));
-        }
-        lu[st] = a;
-    }
-    __syncwarp();
-    const int* pd = M::gw_piv_diag();
-    const int* lsp = M::gw_lsc_ptr();
-    const int* lst = M::gw_lsc_st();
-    const int* upp = M::gw_up_ptr();
-    const int* uij = M::gw_up_ij();
-    const int* uik = M::gw_up_ik();
-    const int* ukj = M::gw_up_kj();
-    for (int k = 0; k < M::ISCHAN; ++k) {
-        const double v = 1.0 / lu[pd[k]];
-        vd[k] = v;
-        for (int t = lsp[k] + lane; t < lsp[k + 1]; t += 32) lu[lst[t]] = lu[lst[t]] * v;
-        __syncwarp();
-        for (int t = upp[k] + lane; t < upp[k + 1]; t += 32) lu[uij[t]] = fma(-lu[uik[t]], lu[ukj[t]], lu[uij[t]]);
-        __syncwarp();
-    }
-}
-
-// forward then backward substitution in place at ws[rhs], rows of a dependency level over
-// the lanes, each row's terms in RBSOLVE's order
-template <class M>
-__device__ void coop_solve(double* __restrict__ ws, int rhs)
-{
-    const int lane = threadIdx.x & 31;
-    const double* __restrict__ lu = ws + M::OFF_LU;
-    const double* __restrict__ vd = ws + M::OFF_VDIAG;
-    double* __restrict__ b = ws + rhs;
-    const int* flp = M::gw_fl_ptr();
-    const int* flr = M::gw_fl_row();
-    const int* frp = M::gw_fr_ptr();
-    const int* frs = M::gw_fr_st();
-    const int* frc = M::gw_fr_col();
-    for (int l = 0; l < M::GW_NFL; ++l) {
-        for (int u = flp[l] + lane; u < flp[l + 1]; u += 32) {
-            const int i = flr[u];
-            double x = b[i];
-            for (int t = frp[i]; t < frp[i + 1]; ++t) x = fma(-lu[frs[t]], b[frc[t]], x);
-            b[i] = x;
-        }
-        __syncwarp();
-    }
-    const int* blp = M::gw_bl_ptr();
-    const int* blr = M::gw_bl_row();
-    const int* brp = M::gw_br_ptr();
-    const int* brs = M::gw_br_st();
-    const int* brc = M::gw_br_col();
-    for (int l = 0; l < M::GW_NBL; ++l) {
-        for (int u = blp[l] + lane; u < blp[l + 1]; u += 32) {
-            const int i = blr[u];
-            double x = b[i];
-            for (int t = brp[i]; t < brp[i + 1]; ++t) x = fma(-lu[brs[t]], b[brc[t]], x);
-            b[i] = x * vd[i];
-        }
-        __syncwarp();
-    }
+    SYNC();
 }
 
 // The f evaluation a cell asked for, with its predictor matrix first and its corrector
 // solve after (day pattern, see the file comment).
-template <class M, int S, bool COOP>
+template <class M, int S>
 __device__ __forceinline__ void evaluate(double* __restrict__ ws, const State& s, bool go)
 {
+    constexpr bool COOP = false;
     if (go && s.need_jac) {
-        if (COOP) {
-            coop_pdecomp<M>(ws, s.r1delt);
-        } else {
-            M::gear_explic_0(ws);
-            M::gear_pdecomp_0(ws, s.r1delt);
-        }
+        M::gear_explic_0(ws);
+        M::gear_pdecomp_0(ws, s.r1delt);
     }
     if (go) {
-        if (COOP) coop_feval<M>(ws);
-        else M::feval_0(ws, M::GEAR_CNEW, M::GEAR_GLOSS);
-        SYNC();
-        LOOP(i, M::ISCHAN) {   // SUBFUN's floor (grsubfun.F:164-171)
-            double& g = GW(M::GEAR_GLOSS + i);
-            if (GW(M::GEAR_CNEW + i) <= ZBOUND && g < 0.0) g = 0.0;
-        }
-        SYNC();
+        M::feval_0(ws, M::GEAR_CNEW, M::GEAR_GLOSS);
+        floor_gloss<M, S, COOP>(ws);
     }
     if (go && s.label == L_ITER_POST) {
-        const double delt = s.delt;
-        LOOP(i, M::ISCHAN) {   // grsmvgear.F:616-620
-            double& g = GW(M::GEAR_GLOSS + i);
-            g = fma(delt, g, -(GW(M::GEAR_CONC + M::ISCHAN + i) + GW(M::GEAR_DTLOS + i)));
-        }
-        SYNC();
-        if (COOP) coop_solve<M>(ws, M::GEAR_GLOSS);
-        else M::solve_0(ws, M::GEAR_GLOSS);
-        SYNC();
+        corrector_rhs<M, S, COOP>(ws, s.delt);
+        M::solve_0(ws, M::GEAR_GLOSS);
     }
 }
 #undef REDUCE_SQ
@@ -886,7 +749,7 @@ __global__ void __launch_bounds__(GEAR_WPB * 32, GEAR_WARPS_PER_SM / GEAR_WPB) k
             cell = -1;
             busy = false;
         }
-        gear::evaluate<M, 32, false>(ws, s, busy);
+        gear::evaluate<M, 32>(ws, s, busy);
     }
     if (a.counters) {
         for (int o = 16; o > 0; o >>= 1) {
@@ -903,85 +766,6 @@ __global__ void __launch_bounds__(GEAR_WPB * 32, GEAR_WARPS_PER_SM / GEAR_WPB) k
             atomicAdd(&a.counters[3], sunlit);
             atomicAdd(&a.counters[4], sun_att);
         }
-    }
-}
-
-// One cell per warp, the cell's workspace in shared memory (GEAR_WS_ELEMS doubles,
-// stride 1; dynamic shared memory of that size per one-warp block): the lanes share the
-// cell's element-wise work, f evaluation, LU and solves.  SMVGEAR's stiffest cells need
-// tens of thousands of Newton iterations in one call, a call lasts as long as its slowest
-// cell, and on this GPU one FP64 warp instruction takes 64 cycles whatever its number of
-// active lanes, so a lone cell must spread its FP64 work over the lanes to advance.
-// Cells come from the work queue; results equal k_gear's bit for bit.
-template <class M, bool GRID>
-__global__ void __launch_bounds__(32) k_gear_warp(GridArgs a, QueueArgs q, GearArgs g)
-{
-    extern __shared__ double sm[];
-    const int lane = threadIdx.x & 31;
-    // lane 0's slot of this warp's global workspace, for the gather (stride 32)
-    double* wsg = a.ws + (size_t)blockIdx.x * ((size_t)M::WS_ELEMS * 32);
-    const gear::Coef* K = g.coef;
-    const unsigned long long qlen = queue_len(q, a.ncell);
-    unsigned long long acc = 0, rej = 0, failed = 0, sunlit = 0, sun_att = 0;
-    for (;;) {
-        unsigned long long pos = 0;
-        if (lane == 0) pos = atomicAdd(q.head, 1ull);
-        pos = __shfl_sync(0xffffffffu, pos, 0);
-        if (pos >= qlen) break;
-        const long long cell = q.cell0 + (q.order ? q.order[pos] : (long long)pos);
-        bool sun;
-        if (GRID) {
-            int sflag = 0;
-            if (lane == 0) sflag = gather_cell<M>(a, cell, wsg, true) ? 1 : 0;
-            sun = __shfl_sync(0xffffffffu, sflag, 0) != 0;
-            __syncwarp();
-            for (int i = lane; i < M::NSPEC; i += 32) sm[M::GEAR_CNEW + i] = wsg[(M::OFF_Y + i) * 32];
-            for (int r = lane; r < M::NRXNS; r += 32) sm[M::OFF_RKI + r] = wsg[(M::OFF_RKI + r) * 32];
-        } else {
-            for (int i = lane; i < M::NSPEC; i += 32) sm[M::GEAR_CNEW + i] = g.y[(size_t)i * a.ncell + cell];
-            for (int r = lane; r < M::NRXNS; r += 32) sm[M::OFF_RKI + r] = g.rk[(size_t)r * a.ncell + cell];
-            sun = g.night[cell] == 0;
-        }
-        __syncwarp();
-        gear::State s;
-        gear::start<M, 1, true>(s, sm, sun, K, GRID && a.yave != nullptr);
-        while (gear::advance<M, 1, true>(sm, s, K, a.chemstep) == gear::NEED_F)
-            gear::evaluate<M, 1, true>(sm, s, true);
-        if (GRID) {   // write-back as scatter_cell
-            const double densd = (double)a.dens[cell];
-            for (int i = lane; i < M::ISCHAN; i += 32) {
-                const int old = M::inew2old(i);
-                const double y = sm[M::GEAR_CNEW + i];
-                const float v = a.convert[old] ? (float)((a.rev_conv[old] * densd) * y) : (float)y;
-                a.cgrid[(size_t)a.cgrid_index[old] * a.ncell + cell] = v;
-                if (a.yave) a.yave[(size_t)i * a.ncell + cell] = sm[M::GEAR_CAVEG + i];
-            }
-        } else {
-            for (int i = lane; i < M::NSPEC; i += 32) g.y[(size_t)i * a.ncell + cell] = sm[M::GEAR_CNEW + i];
-            if (g.cell_stats && lane == 0) {
-                int* o = g.cell_stats + (size_t)8 * cell;
-                o[0] = s.st.nsteps; o[1] = s.st.ncfail; o[2] = s.st.nefail; o[3] = s.st.npderiv;
-                o[4] = s.st.nsubfun; o[5] = s.st.nnewt; o[6] = s.st.maxord; o[7] = s.st.status;
-            }
-        }
-        __syncwarp();   // the next cell overwrites the shared workspace
-        if (lane == 0) {
-            const int att = s.st.nsteps + s.st.ncfail + s.st.nefail;
-            acc += s.st.nsteps;
-            rej += s.st.ncfail + s.st.nefail;
-            failed += s.st.status != gear::ST_OK;
-            sunlit += s.lsun;
-            if (s.lsun) sun_att += att;
-            if (a.cell_status) a.cell_status[cell] = s.st.status;
-            if (a.cell_steps) a.cell_steps[cell] = att;
-        }
-    }
-    if (a.counters && lane == 0) {
-        atomicAdd(&a.counters[0], acc);
-        atomicAdd(&a.counters[1], rej);
-        atomicAdd(&a.counters[2], failed);
-        atomicAdd(&a.counters[3], sunlit);
-        atomicAdd(&a.counters[4], sun_att);
     }
 }
 

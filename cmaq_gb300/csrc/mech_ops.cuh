@@ -11,6 +11,7 @@
 #include "gear.cuh"
 #include "coop.cuh"
 #include "ebi_coop.cuh"
+#include "gear_coop.cuh"
 
 struct MechOps {
     const char* name;
@@ -191,14 +192,14 @@ struct MechOps {
         *bps = a < b ? a : b;                                                                       \
         return e;                                                                                   \
     }                                                                                               \
-    size_t gearw_smem_() { return (size_t)T_::GEAR_WS_ELEMS * sizeof(double); }                     \
+    size_t gearw_smem_() { return coop::smem_bytes<NS::CoopGear>(1); }                              \
     template <bool G>                                                                               \
     cudaError_t gearw_attr_()                                                                       \
     {                                                                                               \
-        cudaError_t r = cudaFuncSetAttribute(chem::k_gear_warp<T_, G>,                              \
+        cudaError_t r = cudaFuncSetAttribute(chem::k_gear_warp<T_, NS::CoopGear, G>,                              \
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gearw_smem_()); \
         if (r != cudaSuccess) return r;                                                             \
-        return cudaFuncSetAttribute(chem::k_gear_warp<T_, G>, cudaFuncAttributePreferredSharedMemoryCarveout, \
+        return cudaFuncSetAttribute(chem::k_gear_warp<T_, NS::CoopGear, G>, cudaFuncAttributePreferredSharedMemoryCarveout, \
                                     (int)cudaSharedmemCarveoutMaxShared);                           \
     }                                                                                               \
     cudaError_t gear_warp_(const chem::GridArgs& a, const chem::QueueArgs& q, const chem::GearArgs& g, bool grid, \
@@ -206,8 +207,8 @@ struct MechOps {
     {                                                                                               \
         cudaError_t r = grid ? gearw_attr_<true>() : gearw_attr_<false>();                          \
         if (r != cudaSuccess) return r;                                                             \
-        if (grid) chem::k_gear_warp<T_, true><<<nb, 32, gearw_smem_(), s>>>(a, q, g);               \
-        else chem::k_gear_warp<T_, false><<<nb, 32, gearw_smem_(), s>>>(a, q, g);                   \
+        if (grid) chem::k_gear_warp<T_, NS::CoopGear, true><<<nb, 32, gearw_smem_(), s>>>(a, q, g);               \
+        else chem::k_gear_warp<T_, NS::CoopGear, false><<<nb, 32, gearw_smem_(), s>>>(a, q, g);                   \
         return cudaGetLastError();                                                                  \
     }                                                                                               \
     cudaError_t gear_warp_occupancy_(int* bps)                                                      \
@@ -216,9 +217,9 @@ struct MechOps {
         if (r == cudaSuccess) r = gearw_attr_<false>();                                             \
         if (r != cudaSuccess) return r;                                                             \
         int a = 0, b = 0;                                                                           \
-        r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, chem::k_gear_warp<T_, true>, 32, gearw_smem_()); \
+        r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, chem::k_gear_warp<T_, NS::CoopGear, true>, 32, gearw_smem_()); \
         if (r != cudaSuccess) return r;                                                             \
-        r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, chem::k_gear_warp<T_, false>, 32, gearw_smem_()); \
+        r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, chem::k_gear_warp<T_, NS::CoopGear, false>, 32, gearw_smem_()); \
         *bps = a < b ? a : b;                                                                       \
         return r;                                                                                   \
     }                                                                                               \

@@ -93,3 +93,22 @@ def test_ebi_cells_that_reach_the_iteration_cap():
     s.set_tuning(ebi_warp=0)
     assert 0 < a[1][0]["failed_cells"] < 130
     same(run(s, t, -1, 1), a)
+
+
+@pytest.mark.parametrize("mech,dims", [("cb6r5_ae7_aq", (1, 1, 1)), ("cb6r5_ae7_aq", (13, 4, 2)),
+                                       ("cracmm2", (5, 4, 1))])
+def test_gear_same_bits_as_one_cell_per_lane(mech, dims):
+    _, t, s = setup(mech, dims, seed=37, solver="gear")
+    s.set_tuning(gear_warp=1)
+    a = run(s, t, -1)
+    s.set_tuning(gear_warp=0)
+    same(run(s, t, -1), a)
+
+
+def test_gear_cells_that_reach_the_evaluation_cap():
+    _, t, s = setup("cb6r5_ae7_aq", (9, 5, 2), seed=38, solver="gear", max_iter=150)
+    s.set_tuning(gear_warp=1)
+    a = run(s, t, -1, 1)
+    s.set_tuning(gear_warp=0)
+    assert 0 < a[1][0]["failed_cells"] < 90
+    same(run(s, t, -1, 1), a)
