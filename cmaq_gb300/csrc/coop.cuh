@@ -248,12 +248,13 @@ static __device__ __noinline__ void special_row(uint2 w, uint32_t cell, uint32_t
     sts_if(cell + (w.y & 0xfff8u), w.y & D_STORE, r);
 }
 
-// The rows of a program on the warp's cell; every warp of the block calls it (S: Stream or Feed).  While row t's FMA is under way, row t - 1's results are stored and then the
+// The rows of a program on the warp's cell; every warp of the block calls it (S: Stream or Feed;
+// on, the same in all lanes: false to stay with the block without going through the rows).  While row t's FMA is under way, row t - 1's results are stored and then the
 // operands of row t + 2 loaded, so that a row waits for neither (with the operands of row
 // t + 1 loaded there it waited for them: 135 cycles a row); the schedule knows that a row's
 // results can be loaded three rows later.
 template <class C, class S>
-__device__ __forceinline__ void run(S& st, int rows, uint32_t cell, uint32_t cst)
+__device__ __forceinline__ void run(S& st, int rows, uint32_t cell, uint32_t cst, bool on = true)
 {
     constexpr int W = 32;
     double acc = 0.0;
@@ -262,7 +263,7 @@ __device__ __forceinline__ void run(S& st, int rows, uint32_t cell, uint32_t cst
         uint32_t p = st.wait() + (threadIdx.x & 31) * 8;
         __syncwarp();
         uint32_t pending = 0;   // word 1 of the row whose result acc has not been stored yet
-        if (st.ok) {
+        if (st.ok && on) {
             uint2 w = ldw(p), w1 = ldw(p + W * 8), w2 = ldw(p + 2 * W * 8);
             Operands o = operands(w, cell, cst), o1 = operands(w1, cell, cst);
             for (int r = 0; r < nr; r += UNROLL) {   // programs are padded to a multiple of UNROLL rows

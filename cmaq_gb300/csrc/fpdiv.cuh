@@ -103,7 +103,7 @@ FPDIV_HD inline uint32_t recip31(uint32_t hi, uint32_t lo)
 static __device__ __noinline__ double div_hw(double a, double b) { return a / b; }
 #endif
 
-// a / b for operands and result in the normal range; *ok is false otherwise
+// a / b for operands and result in the normal range, or a = +-0; *ok is false otherwise
 FPDIV_HD inline double quotient(double a, double b, bool* ok)
 {
     const uint64_t ua = bits(a), ub = bits(b);
@@ -127,9 +127,10 @@ FPDIV_HD inline double quotient(double a, double b, bool* ok)
     uint64_t q = ((uint64_t)q1 << 24) + q2 + (r2 >= mb ? 2u : 1u);
     q >>= 1;
     const uint32_t e = ea - eb + 1022u - (lt ? 1u : 0u);                 // biased exponent - 1
-    *ok = (ea - 1u < 2046u) && (eb - 1u < 2046u) && e < 2045u;
     const uint32_t sign = (ah ^ bh) & 0x80000000u;
-    return from_bits(((uint32_t)(q >> 32) + (e << 20)) | sign, (uint32_t)q);
+    const bool zero = (ah << 1 | al) == 0u;                              // +-0 / b: exact, and frequent
+    *ok = (eb - 1u < 2046u) && (zero || ((ea - 1u < 2046u) && e < 2045u));
+    return zero ? from_bits(sign, 0u) : from_bits(((uint32_t)(q >> 32) + (e << 20)) | sign, (uint32_t)q);
 }
 
 // a / b

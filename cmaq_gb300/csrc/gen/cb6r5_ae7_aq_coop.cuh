@@ -6,7 +6,7 @@ namespace mech_cb6r5_ae7_aq {
 extern __device__ const double c_coop_const[264];
 extern __device__ const uint2 c_coop_rows[38528];
 extern __device__ const double c_coopebi_const[264];
-extern __device__ const uint2 c_coopebi_rows[8960];
+extern __device__ const uint2 c_coopebi_rows[7168];
 extern __device__ const double c_coopgear_const[264];
 extern __device__ const uint2 c_coopgear_rows[29184];
 struct Coop {
@@ -24,9 +24,9 @@ struct CoopEbi {
     static constexpr int ELEMS = 2464, NCONST = 264, MAX_CELLS = 10;
     static constexpr int YC = 0, YC0 = 149, YCP = 298, PROD = 447, LOSS = 596, PNEG = 745, RKI = 894, DTC = 1592, Z = 1593, ONE = 1594;
     static constexpr int CHUNK = 28, TABLE_SMEM = 15936;
-    static constexpr int ITERATION_ROWS = 256;
+    static constexpr int ITERATION_ROWS = 216;
     // chunks of one pass through the programs (iteration), and where each lies
-    static constexpr int PASS = 10;
+    static constexpr int PASS = 8;
     static __device__ __forceinline__ int chunk(int k) { return k; }
     static __device__ __forceinline__ const double* constants() { return c_coopebi_const; }
     static __device__ __forceinline__ const uint2* rows() { return c_coopebi_rows; }

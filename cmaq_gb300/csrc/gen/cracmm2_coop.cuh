@@ -6,7 +6,7 @@ namespace mech_cracmm2 {
 extern __device__ const double c_coop_const[544];
 extern __device__ const uint2 c_coop_rows[69888];
 extern __device__ const double c_coopebi_const[550];
-extern __device__ const uint2 c_coopebi_rows[14336];
+extern __device__ const uint2 c_coopebi_rows[13440];
 extern __device__ const double c_coopgear_const[544];
 extern __device__ const uint2 c_coopgear_rows[57088];
 struct Coop {
@@ -24,9 +24,9 @@ struct CoopEbi {
     static constexpr int ELEMS = 3067, NCONST = 550, MAX_CELLS = 8;
     static constexpr int YC = 0, YC0 = 189, YCP = 378, PROD = 567, LOSS = 756, PNEG = 945, RKI = 1134, DTC = 2196, Z = 2197, ONE = 2198;
     static constexpr int CHUNK = 28, TABLE_SMEM = 15936;
-    static constexpr int ITERATION_ROWS = 440;
+    static constexpr int ITERATION_ROWS = 416;
     // chunks of one pass through the programs (iteration), and where each lies
-    static constexpr int PASS = 16;
+    static constexpr int PASS = 15;
     static __device__ __forceinline__ int chunk(int k) { return k; }
     static __device__ __forceinline__ const double* constants() { return c_coopebi_const; }
     static __device__ __forceinline__ const uint2* rows() { return c_coopebi_rows; }

@@ -2,8 +2,6 @@
 // constants (aqchem_kmt.F90:371-396), rate constants (aqchem_Initialize.F90:491-636,
 // aqchem_Rates.F90:456-579), tolerances, Fun, Jac_SP, KppDecomp, KppSolve as straight-line
 // code.  Included inside namespace kmt2 by csrc/kmt2.cuh.  Do not edit.
-#pragma once
-
 KQ_HD inline void kq_henry(Cell& c, float t2)
 {
     c.henry[0] = (double)kq_hlconst((float)0x1.6666660000000p+0, (float)0x1.6a80000000000p+11, t2);   // SO2H
@@ -481,6 +479,7 @@ KQ_HD inline void kq_add_diagonal(double* g, double x)
     g[737 * KQ_S] = g[737 * KQ_S] + x;
 }
 
+#if KMT2_STRIDE != 1   // with stride 1 they are the cooperative kernels' programs
 KQ_HD KQ_NOINLINE void kqu_fun_0(const double* v, const double* f, const double* r, double* vdot)
 {
     vdot[0 * KQ_S] = 0.0 - (r[32 * KQ_S] * v[0 * KQ_S]);
@@ -3336,3 +3335,4 @@ KQ_HD inline void kqu_solve(const double* jvs, double* x)
     kqu_solve_b1(jvs, x);
     kqu_solve_b2(jvs, x);
 }
+#endif

@@ -20,6 +20,7 @@
 
 #include "../../include/cmaqchem.h"
 #include "kmt2.cuh"
+#include "kmt2_coop.cuh"
 
 __attribute__((visibility("hidden"))) void cmaqchem_set_error(const std::string& msg);
 
@@ -196,10 +197,73 @@ __global__ void __launch_bounds__(KMT2_THREADS, KMT2_MIN_BLOCKS) k_aqchem_queue(
         });
 }
 
+// The same calls, one cell per warp (kmt2_coop.cuh)
+__global__ void __launch_bounds__(kmt2_coop::Coop::MAX_CELLS * 32, 1) k_kmt2_coop(Kmt2Args a)
+{
+    extern __shared__ __align__(128) char smem[];
+    using namespace kmt2w;
+    const long long n = a.ncell;
+    kmt2_coop::integrate(
+        smem, a.next, n,
+        [&](long long cell, Cell& c, double* ws) {
+            return kq_setup(c, a.params + cell, n, a.var_mix + cell, n, a.params[P_HO * n + cell], ws + W_Y, ws + W_F,
+                            ws + W_R);
+        },
+        [&](long long cell, const Cell&, const Lane& L, const long long* st, const double* ws) {
+            const int lane = threadIdx.x & 31;
+            const bool nan = L.ierr <= -101;   // failed set-up: no state to return
+            for (int i = lane; i < NVAR; i += 32) a.var_out[i * n + cell] = nan ? (double)NAN : ws[W_Y + i];
+            if (a.fix_out && lane < NFIX) a.fix_out[lane * n + cell] = nan ? (double)NAN : ws[W_F + lane];
+            if (lane == 0)
+                for (int i = 0; i < NSTAT; ++i) a.stats[i * n + cell] = (int)st[i];
+        });
+}
+
+__global__ void __launch_bounds__(kmt2_coop::Coop::MAX_CELLS * 32, 1) k_aqchem_coop(AqchemArgs a)
+{
+    extern __shared__ __align__(128) char smem[];
+    using namespace kmt2w;
+    const long long n = a.ncell;
+    kmt2_coop::integrate(
+        smem, a.next, n,
+        [&](long long cell, Cell& c, double* ws) {
+            kq_aq_map(a.params + cell, a.gas + cell, a.aer + cell, a.naer, a.ai, a.fac, n, ws);
+            return kq_setup(c, a.params + cell, n, ws + W_YNEW, KQ_S, a.gas[KG_HO * n + cell], ws + W_Y, ws + W_F,
+                            ws + W_R);
+        },
+        [&](long long cell, const Cell& c, const Lane& L, const long long* st, const double* ws) {
+            if ((threadIdx.x & 31) == 0)
+                kq_aq_finish(c, L.ierr, st, a.params + cell, a.gas + cell, a.aer + cell, a.naer, a.ai, a.fac,
+                             a.gas_wdep + cell, a.aer_wdep + cell, a.out + cell, a.stats + cell, n, ws);
+        });
+}
+
 int fail(const std::string& msg)
 {
     cmaqchem_set_error(msg);
     return -1;
+}
+
+// Whether a call takes the cooperative kernels (same results): 333 cells take 12.8 ms there and
+// 148 one cell per lane, 4,000 cells 40 and 165 ms, 25,000 cells 225 and 277 ms; at 100,000 cells
+// the lanes are full: 880 and 661 ms.
+constexpr long long COOP_LIMIT = 35000;
+bool use_coop(long long ncell) { return ncell <= COOP_LIMIT; }
+
+template <class Args>
+cudaError_t launch_coop(void (*kernel)(Args), const Args& a, cudaStream_t s)
+{
+    int dev = 0, nsm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    const int cells = (int)std::min<long long>(kmt2_coop::Coop::MAX_CELLS, (a.ncell + nsm - 1) / nsm);
+    const int nb = (int)std::min<long long>(nsm, (a.ncell + cells - 1) / cells);
+    const size_t bytes = coop::smem_bytes<kmt2_coop::Coop>(cells);
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) return e;
+    kernel<<<nb, cells * 32, bytes, s>>>(a);
+    return cudaGetLastError();
 }
 
 // Lanes of a call: whole warps of the workspace (at most enough for ncell), the queue
@@ -250,8 +314,12 @@ extern "C" int cmaqchem_kmt2_solve_device(long long ncell, const double* params,
     cudaError_t e = cudaMemsetAsync(next, 0, sizeof(unsigned long long), s);
     if (e != cudaSuccess) return fail(std::string("queue counter: ") + cudaGetErrorString(e));
     Kmt2Args a{params, var_mix, var_out, fix_out, stats, workspace, next, ncell, nlanes};
-    k_kmt2_queue<<<(unsigned)blocks, KMT2_THREADS, 0, s>>>(a);
-    e = cudaGetLastError();
+    if (use_coop(ncell)) {
+        e = launch_coop(k_kmt2_coop, a, s);
+    } else {
+        k_kmt2_queue<<<(unsigned)blocks, KMT2_THREADS, 0, s>>>(a);
+        e = cudaGetLastError();
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(std::string("k_kmt2_queue: ") + cudaGetErrorString(e));
     return 0;
@@ -335,8 +403,12 @@ extern "C" int cmaqchem_aqchem_device(long long ncell, const double* params, dou
     a.ncell = ncell;
     a.nlanes = nlanes;
     a.naer = naer;
-    k_aqchem_queue<<<(unsigned)blocks, KMT2_THREADS, 0, s>>>(a);
-    e = cudaGetLastError();
+    if (use_coop(ncell)) {
+        e = launch_coop(k_aqchem_coop, a, s);
+    } else {
+        k_aqchem_queue<<<(unsigned)blocks, KMT2_THREADS, 0, s>>>(a);
+        e = cudaGetLastError();
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(std::string("k_aqchem_queue: ") + cudaGetErrorString(e));
     return 0;

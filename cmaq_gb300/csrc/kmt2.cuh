@@ -22,7 +22,9 @@
 // lane-interleaved FP64 workspace (element i of a lane at ws[i * KQ_S]); inputs and
 // outputs are [element][cell] with stride n.  The header compiles as plain C++ too, so
 // the host can run exactly this code.
-#pragma once
+//
+// It may be included again with KMT2_NS and KMT2_STRIDE redefined: kmt2_coop.cuh takes the
+// scalar parts (set-up, rate laws, mapping) for a workspace of one cell, stride 1.
 
 #include <float.h>
 #include <math.h>
@@ -35,14 +37,19 @@
 #define KQ_NOINLINE
 #endif
 
-namespace kmt2 {
+#ifndef KMT2_NS
+#define KMT2_NS kmt2
+#define KMT2_STRIDE 32
+#endif
+
+namespace KMT2_NS {
 
 #include "gen/kmt2_aq_consts.cuh"
 
 // The workspace holds a warp's 32 lanes side by side: element i of a lane at ws[i * KQ_S]
 // (ws pointing at the lane's first element), so a warp's access to one element reads 256
 // consecutive bytes and every offset is a constant.
-constexpr long long KQ_S = 32;
+constexpr long long KQ_S = KMT2_STRIDE;
 
 // per-cell parameters, [KQ_NPARAM][ncell] (include/cmaqchem.h: CMAQCHEM_KMT2_*)
 enum { P_TEMP2 = 0, P_PRES_PA, P_TAUCLD, P_PRCRATE, P_WCAVG, P_WTAVG, P_AIRM, P_ALFA0, P_ALFA3, P_COSZEN,
@@ -166,9 +173,13 @@ KQ_HD inline double kq_kphot(const Cell& c, double maxc, double jval)
     return c.czen > 0.001 ? c.photo * 2.718281828 * maxc * kq_exp(-1.0 / c.czen) : 0.0;
 }
 // aqchem_Rates.F90:146-158
+KQ_HD inline double kq_disf_t(const Cell& c, double keq, double dh, double kb)   // its temperature factor
+{
+    return kb * (keq * kq_exp(dh * c.delinvt));
+}
 KQ_HD inline double kq_disf(const Cell& c, double keq, double dh, double kb, int g1)
 {
-    const double k = kb * (keq * kq_exp(dh * c.delinvt));
+    const double k = kq_disf_t(c, keq, dh, kb);
     return g1 == 1 ? k * c.gm1 : k;
 }
 // aqchem_Rates.F90:160-174
@@ -191,12 +202,18 @@ KQ_HD inline double kq_diffusion_factor(const Cell& c, double krate)
     const double q = 3.0 * ((coth / q1) - (1.0 / (q1 * q1)));
     return q > 1.0 ? 1.0 : q;
 }
-// aqchem_Rates.F90:176-249
-KQ_HD inline double kq_krxn(const Cell& c, const double* v, double kr, double dh, int rtype, int qy,
-                            int metal)
+// aqchem_Rates.F90:176-249: the first-order rate that diffusion limits, from its temperature
+// factors e1, e2, e3; then the rate constant from KR * EXP( DH * DELINVT )
+KQ_HD inline double kq_kt_qy(const Cell& c, const double* v, double e1, double e2, double e3)
+{
+    const double k1 = 2.4e+4 * e1;
+    const double k2 = 3.7e+5 * e2;
+    const double k3 = 1.5e+9 * e3;
+    return (k1 * v[L_SO2 * KQ_S] + k2 * v[L_HSO3MIN * KQ_S] + k3 * v[L_SO3MIN2 * KQ_S]) * c.phi2;
+}
+KQ_HD inline double kq_krxn_k(const Cell& c, const double* v, double k, int rtype, int metal)
 {
     const double phi2 = c.phi2;
-    double k = kr * kq_exp(dh * c.delinvt);
     if (rtype == 1) k = (k / (1.0 + 13.0 * v[L_HPLUS * KQ_S] * phi2)) * phi2;
     else if (rtype == 3) k = k * phi2;
     else if (rtype == 4) k = k / phi2;
@@ -204,23 +221,25 @@ KQ_HD inline double kq_krxn(const Cell& c, const double* v, double kr, double dh
         const double s6 = (v[L_H2SO4 * KQ_S] + v[L_HSO4MIN * KQ_S] + v[L_SO4MIN2 * KQ_S]) * phi2;
         k = k / (1.0 + 75.0 * kq_rpow(s6, 0.67));
     }
-    if (qy >= 1) {
-        const double k1 = 2.4e+4 * kq_exp(0.0 * c.delinvt);
-        const double k2 = 3.7e+5 * kq_exp(-5530.88 * c.delinvt);
-        const double k3 = 1.5e+9 * kq_exp(-5280.56 * c.delinvt);
-        const double kt = (k1 * v[L_SO2 * KQ_S] + k2 * v[L_HSO3MIN * KQ_S] + k3 * v[L_SO3MIN2 * KQ_S]) * phi2;
-        k = k * kq_diffusion_factor(c, kt);
-    }
-    return k * phi2;
+    return k;
 }
-// aqchem_Rates.F90:251-362
-KQ_HD inline double kq_kiepox(const Cell& c, const double* v, const double* f, double kh, double khso4,
-                              int type)
+KQ_HD inline double kq_krxn(const Cell& c, const double* v, double kr, double dh, int rtype, int qy,
+                            int metal)
+{
+    double k = kq_krxn_k(c, v, kr * kq_exp(dh * c.delinvt), rtype, metal);
+    if (qy >= 1)
+        k = k * kq_diffusion_factor(c, kq_kt_qy(c, v, kq_exp(0.0 * c.delinvt), kq_exp(-5530.88 * c.delinvt),
+                                                kq_exp(-5280.56 * c.delinvt)));
+    return k * c.phi2;
+}
+// aqchem_Rates.F90:251-362: the first-order rate of the IEPOX reactions; kiepox: the rate
+// constant before the diffusion limitation
+KQ_HD inline double kq_kt_iepox(const Cell& c, const double* v, const double* f, double kh, double khso4, int type,
+                                double* kiepox)
 {
     const double phi2 = c.phi2;
-    if (c.ispc8 <= 0 ? type > 0 : type < 1) return 0.0;
     const double h = v[L_HPLUS * KQ_S], hso4 = v[L_HSO4MIN * KQ_S], so4 = v[L_SO4MIN2 * KQ_S];
-    double kiepox = kh * h * phi2 + khso4 * hso4 * phi2;
+    *kiepox = kh * h * phi2 + khso4 * hso4 * phi2;
     double kt = (9.0e-4 * h * phi2 + 1.31e-5 * hso4 * phi2) * f[L_H2O * KQ_S] * phi2;
     if (type <= 1) {
         kt = kt + (8.83e-3 * h * phi2 + 2.92e-6 * hso4 * phi2) * so4 * phi2;
@@ -234,13 +253,22 @@ KQ_HD inline double kq_kiepox(const Cell& c, const double* v, const double* f, d
     } else {
         kt = kt + (2.0e-4 * h * phi2 + 2.92e-6 * hso4 * phi2) * so4 * phi2;
     }
+    return kt;
+}
+KQ_HD inline bool kq_iepox_off(const Cell& c, int type) { return c.ispc8 <= 0 ? type > 0 : type < 1; }
+KQ_HD inline double kq_kiepox(const Cell& c, const double* v, const double* f, double kh, double khso4,
+                              int type)
+{
+    if (kq_iepox_off(c, type)) return 0.0;
+    double kiepox;
+    const double kt = kq_kt_iepox(c, v, f, kh, khso4, type, &kiepox);
     kiepox = kiepox * kq_diffusion_factor(c, kt);
-    return kiepox * phi2;
+    return kiepox * c.phi2;
 }
 
 // ionic strength and activity coefficients (aqchem_Rates.F90:423-452), terms in the
 // reference's order (L_HMSMIN twice, as there)
-KQ_HD KQ_NOINLINE void kq_ionic(Cell& c, const double* v)
+KQ_HD KQ_NOINLINE double kq_log_gm1(Cell& c, const double* v)   // sets STION, returns LOG10( GM1 )
 {
 #define V(n) v[(n) * KQ_S]
     const double sum = V(L_HPLUS) + V(L_NH4PLUS) + V(L_OHMIN) + V(L_HCO3MIN) + V(L_O2MIN) + V(L_NO2MIN)
@@ -253,7 +281,11 @@ KQ_HD KQ_NOINLINE void kq_ionic(Cell& c, const double* v)
                      + 9.0 * V(L_FEPLUS3);
 #undef V
     c.stion = 0.5 * sum * c.phi2;
-    const double lg1 = -0.509 * (sqrt(c.stion) / (1.0 + sqrt(c.stion)) - 0.2 * c.stion);
+    return -0.509 * (sqrt(c.stion) / (1.0 + sqrt(c.stion)) - 0.2 * c.stion);
+}
+KQ_HD inline void kq_ionic(Cell& c, const double* v)
+{
+    const double lg1 = kq_log_gm1(c, v);
     c.gm1 = kq_rpow(10.0, lg1);
     const double gm2 = kq_rpow(10.0, lg1 * 4.0);
     c.gm2 = gm2 > 1.0e-30 ? gm2 : 1.0e-30;
@@ -392,6 +424,7 @@ KQ_HD inline void kq_return(Lane& L, int ierr)
 // f(YNEW) + (1/h) K1 - (1/h) K2 - (8/3/h) K3; YNEW + K4 is the new state (M = 2, 0, 1, 1:
 // stage 4's Y + 2 K1 + K3 is stage 3's YNEW + K3, bit for bit).
 
+#if KMT2_STRIDE != 1
 // Moves the lane to its next attempt.  Returns true when the cell is finished: L.ierr is
 // IERR (1 = success, -6 / -7 / -8 from ros_Integrator, -100 for 16 calls, -101 / -102 for a
 // failed set-up), also in st[S_IERR].  Each pass of the loop moves the lane on by one
@@ -594,6 +627,8 @@ KQ_HD inline bool kq_advance(Cell& c, Lane& L, double* ws, long long* st)
         return false;
     }
 }
+
+#endif   // KMT2_STRIDE != 1
 
 // ----------------------------------------------------------------------------- the whole AQCHEM
 // AQCHEM's GAS array in AQ_DATA.F's srggas order (29 species, mol/molV)
@@ -1021,4 +1056,4 @@ KQ_HD inline int kq_aq_finish(const Cell& c, int ierr, const long long* st, cons
 #undef AER
 #undef AWD
 
-}  // namespace kmt2
+}  // namespace KMT2_NS

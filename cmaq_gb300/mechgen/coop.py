@@ -43,8 +43,8 @@ SMEM_MAX = 227 * 1024
 TABLE_SMEM = 2 * (CHUNK + AHEAD) * 32 * 8 + 64   # two chunks in flight, each with rows of zeros, and their barriers
 
 # where an operation's addend comes from: the element itself, the lane's accumulator, -0.0
-# (the exact identity of an addition: a product alone); MULACC: acc * x[b]
-LOAD, KEEP, NEG0, MULACC = range(4)
+# (the exact identity of an addition: a product alone); MULACC: acc * x[b]; LOADACC: acc * x[b] + x[d]
+LOAD, KEEP, NEG0, MULACC, LOADACC = range(5)
 # special operations: 1 / x[b], x[a] / x[b], sqrt(x[b]), fmax(x[a], x[b]), copysign(1, x[b])
 RCP, DIV, SQRT, MAX, SIGN = range(1, 6)
 # encoding: word 0 = offset of a | offset of b << 16, word 1 = offset of d, and flags.
@@ -52,7 +52,7 @@ RCP, DIV, SQRT, MAX, SIGN = range(1, 6)
 # Word 1 of a special operation (A_SPECIAL in word 0) holds its kind in place of the addend's.
 A_SPECIAL, C_LOAD, C_KEEP, C_MULACC = 1, 1, 2, 4
 D_STORE, B_CONST, A_NEG = 1 << 16, 1 << 17, 1 << 31
-ADDEND = {LOAD: C_LOAD, KEEP: C_KEEP, NEG0: 0, MULACC: C_MULACC}
+ADDEND = {LOAD: C_LOAD, KEEP: C_KEEP, NEG0: 0, MULACC: C_MULACC, LOADACC: C_LOAD | C_MULACC}
 
 
 @dataclass
@@ -109,11 +109,14 @@ def schedule(ops, width: int, special_cost: int = 3) -> Schedule:
     preds = dependencies(ops)
     succ = [[] for _ in range(n)]
     chain = [None] * n
+    factor = [None] * n                  # the operation that forms the factor a of a sum's term
     for i, ps in enumerate(preds):
         for p, k in ps:
             succ[p].append((i, k))
             if k == "C":
                 chain[i] = p
+            if k == "R" and ops[i][0] == ops[p][0] == "F" and ops[i][5] == LOAD and ops[p][1] == ops[i][2] != ops[i][3]:
+                factor[i] = p
 
     def latency(p, k, i):
         if k in "WO":
@@ -140,10 +143,10 @@ def schedule(ops, width: int, special_cost: int = 3) -> Schedule:
     store = [True] * n
     rows, t, done = [], 0, 0
 
-    def earliest(i, skip_chain=False):
+    def earliest(i, skip=None):
         e = 0
         for p, k in preds[i]:
-            if not (skip_chain and k == "C"):
+            if (p, k) != skip:
                 e = max(e, when[p] + latency(p, k, i))
         return e
 
@@ -153,8 +156,11 @@ def schedule(ops, width: int, special_cost: int = 3) -> Schedule:
         specials = sorted((i for i in ready if ops[i][0] == "D"), key=lambda i: (-prio[i], i))[:width]
         # operations that a lane can go on with in its accumulator
         goes_on = {i for i in waiting if chain[i] is not None and ops[i][0] == ops[chain[i]][0] == "F"
-                   and lane_acc[lane_of[chain[i]]] == chain[i] and earliest(i, skip_chain=True) <= t}
-        cand = sorted(goes_on.union(i for i in ready if ops[i][0] == "F" and ops[i][5] != MULACC),
+                   and lane_acc[lane_of[chain[i]]] == chain[i] and earliest(i, (chain[i], "C")) <= t}
+        # or whose factor a lane has just formed there
+        takes = {i for i in waiting if factor[i] is not None and i not in goes_on and ready_at[i] > t
+                 and lane_acc[lane_of[factor[i]]] == factor[i] and earliest(i, (factor[i], "R")) <= t}
+        cand = sorted(goes_on.union(takes, (i for i in ready if ops[i][0] == "F" and ops[i][5] != MULACC)),
                       key=lambda i: (-prio[i], i))
         if specials and t % UNROLL == 0 and (not cand or prio[specials[0]] >= prio[cand[0]] - SLACK):
             rows.append(("D", specials + [None] * (width - len(specials))))
@@ -172,11 +178,11 @@ def schedule(ops, width: int, special_cost: int = 3) -> Schedule:
                     break
                 if ops[i][5] == MULACC:
                     continue
-                ln = lane_of[chain[i]] if i in goes_on else None
+                ln = lane_of[chain[i]] if i in goes_on else lane_of[factor[i]] if i in takes else None
                 if ln is not None and lanes[ln] is None and product[ln] is None:
                     lanes[ln] = i
                     room -= 1
-                    kind[i] = KEEP if kind[i] == LOAD else MULACC
+                    kind[i] = LOADACC if i in takes else KEEP if kind[i] == LOAD else MULACC
                 elif ready_at[i] <= t:
                     fresh.append(i)
                     room -= 1
@@ -222,7 +228,7 @@ def encode(ops, sch: Schedule, offset, const_offset, zero: int) -> list[list[tup
                             offset(d) | special | D_STORE | (B_CONST if const else 0)))
                 continue
             k = sch.kind[i]
-            w0 = (zero if k == MULACC else offset(a)) | (const_offset(b[1]) if const else offset(b)) << 16
+            w0 = (zero if k in (MULACC, LOADACC) else offset(a)) | (const_offset(b[1]) if const else offset(b)) << 16
             w1 = (offset(d) | ADDEND[k]) + (D_STORE if sch.store[i] else 0)
             row.append((w0, w1 + (B_CONST if const else 0) + (A_NEG if neg else 0)))
         out.append(row)
@@ -501,16 +507,19 @@ def gear_tables(mech: str, width: int = WIDTH):
 # takes a product and an addition, x * 1.0 + acc, unless its factor is a power of two: such a
 # product is exact, and the fused operation gives the same sum.
 
-_TOKEN = re.compile(r"\s*(?:(\d+\.?\d*(?:e[-+]?\d+)?)|(EBI_\w+)\((\d+)\)|(\w+)|(.))")
+_TOKEN = re.compile(r"\s*(?:(0x[0-9a-f.]+p[-+]?\d+|\d+\.?\d*(?:e[-+]?\d+)?)|(EBI_\w+)\((\d+)\)"
+                    r"|(\w+)\[(\d+) \* KQ_S\]|(\w+)|(.))")
 _EBI_ARRAYS = {"EBI_YC": "C", "EBI_YC0": "B", "EBI_YCP": "P", "EBI_RKI": "R", "EBI_RXRAT": "X", "EBI_PROD": "M",
                "EBI_LOSS": "L", "EBI_PNEG": "N"}
 
 
-def _parse(text: str):
-    """An expression of numbers, elements, + - * /, fmax, sqrt, fabs and copysign as nested tuples."""
+def _parse(text: str, arrays=None):
+    """An expression of numbers, elements, + - * /, fmax, sqrt, fabs and copysign as nested tuples;
+    `arrays`: the elements' prefix per array of the KPP code."""
     toks = []
-    for num, arr, idx, name, ch in _TOKEN.findall(text):
-        toks.append(("num", float(num)) if num else ("el", _EBI_ARRAYS[arr] + idx) if arr else
+    for num, arr, idx, karr, kidx, name, ch in _TOKEN.findall(text):
+        toks.append(("num", float.fromhex(num) if "x" in num else float(num)) if num else
+                    ("el", _EBI_ARRAYS[arr] + idx) if arr else ("el", arrays[karr] + kidx) if karr else
                     ("name", name) if name else (ch, None))
     pos = 0
 
@@ -571,8 +580,9 @@ def _parse(text: str):
 class _Emit:
     """Expressions to operations; temporaries come from a ring of places."""
 
-    def __init__(self, P: Program, temps: int):
+    def __init__(self, P: Program, temps: int, memo: bool = False):
         self.P, self.temps, self.next = P, temps, 0
+        self.memo = {} if memo else None     # products that keep their place (their factors do not change)
 
     def temp(self):
         self.next += 1
@@ -581,6 +591,20 @@ class _Emit:
     @staticmethod
     def exact(v: float) -> bool:
         return v != 0.0 and abs(math.frexp(v)[0]) == 0.5
+
+    @classmethod
+    def reads(cls, e, element) -> bool:
+        return e == ("el", element) or any(cls.reads(x, element) for x in e[1:] if isinstance(x, tuple))
+
+    def product(self, e, d):
+        """A product of elements, factor by factor in d."""
+        if e[1][0] == "*":
+            self.product(e[1], d)
+            self.P.fma(d, None, ("c", e[2][1]) if e[2][0] == "num" else self.operand(e[2]), init=MULACC)
+        elif e[1][0] == "num":
+            self.P.fma(d, self.operand(e[2]), ("c", e[1][1]), init=NEG0)
+        else:
+            self.P.fma(d, self.operand(e[1]), ("c", e[2][1]) if e[2][0] == "num" else self.operand(e[2]), init=NEG0)
 
     def operand(self, e):
         """An element that holds the value of e (constants have no element: see `b`)."""
@@ -604,13 +628,16 @@ class _Emit:
             P.fma(dst, a, ("c", 1.0), neg=True, init=NEG0)
             return dst
         if kind == "*":
+            if self.memo is not None and dst is None:
+                if e not in self.memo:
+                    self.memo[e] = f"p{len(self.memo)}"
+                    self.product(e, self.memo[e])
+                return self.memo[e]
             x, y = e[1], e[2]
             if x[0] == "num":
                 x, y = y, x
             if x[0] == "num":
                 raise ValueError("a product of constants")
-            if x[0] != "el" and y[0] != "num" and y[0] == "el":
-                pass
             a = self.operand(x)
             b = ("c", y[1]) if y[0] == "num" else self.operand(y)
             dst = dst or self.temp()
@@ -621,19 +648,28 @@ class _Emit:
             while e[0] in ("+", "-"):
                 terms.append((e[0], e[2]))
                 e = e[1]
-            acc = self.temp()                # not dst itself, which a later term may read
-            if e[0] == "num" and e[1] == 1.0:
+            terms.reverse()
+            # in dst itself, unless a later term reads it
+            inplace = dst is not None and not any(self.reads(t, dst) for _, t in terms)
+            acc = dst if inplace else self.temp()
+            init = LOAD
+            if e == ("num", 0.0):
+                init = NEG0                  # 0.0 +- x: only the sign of a zero could differ
+            elif e[0] == "num" and e[1] == 1.0:
                 P.fma(acc, "O", ("c", 1.0), init=NEG0)
-            else:
+            elif e != ("el", acc):
                 self.value(e, acc)
-            for sign, t in reversed(terms):
+            for sign, t in terms:
                 neg = sign == "-"
                 if t[0] == "*" and t[1][0] == "num" and self.exact(t[1][1]):
-                    P.fma(acc, self.operand(t[2]), ("c", t[1][1]), neg=neg)
+                    P.fma(acc, self.operand(t[2]), ("c", t[1][1]), neg=neg, init=init)
                 elif t[0] == "num":
-                    P.fma(acc, "O", ("c", t[1]), neg=neg)
+                    P.fma(acc, "O", ("c", t[1]), neg=neg, init=init)
                 else:
-                    P.fma(acc, self.operand(t), ("c", 1.0), neg=neg)
+                    P.fma(acc, self.operand(t), ("c", 1.0), neg=neg, init=init)
+                init = LOAD
+            if inplace:
+                return dst
             if dst is None:
                 return acc
             P.fma(dst, acc, ("c", 1.0), init=NEG0)
@@ -815,12 +851,193 @@ def sources(mech: str) -> dict[str, str]:
     return {f"{mech}_coop.cuh": "\n".join(h) + "\n", f"{mech}_coop.cu": "\n".join(c) + "\n"}
 
 
+# ----------------------------------------------------------------------------- KMT2
+# Fun, Jac_SP, KppDecomp and KppSolve of the aqueous mechanism (gen/kmt2_aq.cuh), products and
+# sums rounded one by one as in the EBI code; a product that several sums use is formed once.
+
+def _kmt2_body(name: str) -> list[str]:
+    """The statements of a routine's parts in order."""
+    text = (PKG / "csrc" / "gen" / "kmt2_aq.cuh").read_text()
+    out = []
+    for m in re.finditer(rf"KQ_HD KQ_NOINLINE (?:void|int) {name}\d+\([^)]*\)\n\{{\n(.*?)\n\}}", text, re.S):
+        out += [x.strip() for x in m.group(1).splitlines()]
+    return out
+
+
+def kmt2_programs() -> dict[str, Program]:
+    """Of one Rodas3 step: fjac (F = Fun(Y), J = Jac(Y)), decomp (G in place), solve (V in place),
+    fun (V = Fun(YNEW = W))."""
+    p = {k: Program() for k in ("fjac", "decomp", "solve", "fun")}
+    for name, v, dst, jac in (("fjac", "Y", "F", True), ("fun", "W", "V", False)):
+        em = _Emit(p[name], 0, memo=True)
+        arrays = {"v": v, "f": "H", "r": "R", "vdot": dst, "jvs": "J"}
+        for line in _kmt2_body("kqu_fun_") + (_kmt2_body("kqu_jac_") if jac else []):
+            lhs, rhs = line.rstrip(";").split(" = ", 1)
+            d, e = _parse(lhs, arrays)[1], _parse(rhs, arrays)
+            if e == ("num", 0.0):
+                p[name].fma(d, "Z", ("c", 1.0), init=NEG0)
+            else:
+                em.value(e, d)
+    em = _Emit(p["decomp"], KMT2_RING)
+    arrays = {"jvs": "G", "x": "V"}
+    for line in _kmt2_body("kqu_decomp_"):
+        if line.startswith(("if (fabs(", "return 0")) or line == "}":
+            continue                       # pivots are tested before the program (as they come in)
+        m = re.match(r"\{ const double a = -jvs\[(\d+) \* KQ_S\] / jvs\[(\d+) \* KQ_S\]; jvs\[(\d+) \* KQ_S\] = -a;$", line)
+        if m:
+            low = f"G{m.group(1)}"
+            if m.group(3) != m.group(1):
+                raise ValueError(line)
+            p["decomp"].special(DIV, low, low, f"G{m.group(2)}")
+            continue
+        lhs, rhs = line.rstrip(";").split(" = ", 1)
+        m = re.fullmatch(r"jvs\[(\d+) \* KQ_S\] \+ a \* jvs\[(\d+) \* KQ_S\]", rhs)
+        if not m or lhs != f"jvs[{m.group(1)} * KQ_S]":
+            raise ValueError(line)
+        t = em.temp()                      # x + a b with a = -L: x - L b
+        p["decomp"].fma(t, low, f"G{m.group(2)}", init=NEG0)
+        p["decomp"].fma(f"G{m.group(1)}", t, ("c", 1.0), neg=True)
+    em = _Emit(p["solve"], KMT2_TEMPS)
+    for line in _kmt2_body("kqu_solve_f") + _kmt2_body("kqu_solve_b"):
+        lhs, rhs = line.rstrip(";").split(" = ", 1)
+        d, e = _parse(lhs, arrays)[1], _parse(rhs, arrays)
+        if e[0] == "/":
+            if e[1] != ("el", d):
+                em.value(e[1], d)
+            p["solve"].special(DIV, d, d, em.operand(e[2]))
+        else:
+            em.value(e, d)
+    return p
+
+
+KMT2_TEMPS, KMT2_RING = 288, 640
+
+
+class Kmt2Layout:
+    """Offsets of the one-cell workspace: kmt2.cuh's with stride 1 (Y, YNEW, FCN0, K1-K4, JAC0, GHIMJ, R,
+    FIX), then the temperature factors, the cell's scalars and temporaries.  K4 is the vector
+    that is solved for; products of fjac and decomp lie over YNEW and the stage vectors."""
+
+    def __init__(self, nvar, nlu, nreact, nfix, nfactor, ncell):
+        self.at = {}
+        y, w, f, k = 0, nvar, 2 * nvar, 3 * nvar
+        jac = 7 * nvar
+        g, r, h = jac + nlu, jac + 2 * nlu, jac + 2 * nlu + nreact
+        for v, off, n in (("Y", y, nvar), ("W", w, nvar), ("F", f, nvar), ("V", k + 3 * nvar, nvar), ("J", jac, nlu),
+                          ("G", g, nlu), ("R", r, nreact), ("H", h, nfix)):
+            self.at.update({f"{v}{i}": off + i for i in range(n)})
+        off = h + nfix
+        self.ws_elems = off
+        self.factor, off = off, off + nfactor
+        self.cell, off = off, off + ncell
+        self.temps, off = off, off + KMT2_TEMPS
+        self.at.update(Z=off, O=off + 1)
+        self.elems = off + 2
+        own = list(range(self.temps, self.temps + KMT2_TEMPS))
+        over = list(range(w, w + nvar)) + list(range(k, k + 4 * nvar))
+        self.place = {"fjac": over + own, "decomp": over, "solve": own, "fun": own}
+
+
+def kmt2_rates() -> list[tuple]:
+    """Update_RCONST's rates: (kind, r, integer arguments, real arguments), like kinds together."""
+    text = (PKG / "csrc" / "gen" / "kmt2_aq.cuh").read_text()
+    body = re.search(r"void kq_rates_update\([^)]*\)\n\{\n(.*?)\n\}", text, re.S).group(1)
+    kinds = ("disf", "disb", "krxn", "kiepox")
+    out = []
+    for line in body.splitlines():
+        m = re.fullmatch(r"\s*r\[(\d+) \* KQ_S\] = kq_(\w+)\(c, (?:v, )?(?:f, )?(.*)\);", line)
+        args = [float.fromhex(a) if "x" in a else int(a) for a in m.group(3).split(", ")]
+        ints = [a for a in args if isinstance(a, int)]
+        out.append((kinds.index(m.group(2)), int(m.group(1)), (ints + [0, 0, 0])[:3],
+                    ([a for a in args if isinstance(a, float)] + [0.0, 0.0, 0.0])[:3]))
+    # rates that the aqueous diffusion limits last, those with a power before them: whole rounds of lanes
+    return sorted(out, key=lambda q: (q[0] == 3 or (q[0] == 2 and q[2][1] > 0), q[0] == 2 and q[2][2] > 0, q[0], q[1]))
+
+
+def kmt2_tables(width: int = WIDTH):
+    """(layout, constants, {program: encoded rows})."""
+    consts_text = (PKG / "csrc" / "gen" / "kmt2_aq_consts.cuh").read_text()
+    num = lambda n: int(re.search(rf"constexpr int {n} = (\d+);", consts_text).group(1))
+    progs = kmt2_programs()
+    lay = Kmt2Layout(num("NVAR"), num("LU_NONZERO"), num("NREACT"), num("NFIX"), len(kmt2_rates()), 64)
+    consts = sorted({op[3][1] for p in progs.values() for op in p.ops if isinstance(op[3], tuple)})
+    cof = {c: 8 * q for q, c in enumerate(consts)}
+    tables = {}
+    for name, p in progs.items():
+        ops = place(p.ops, kmt2_places(lay, name, p))
+        tables[name] = encode(ops, schedule(ops, width), lambda e: 8 * e, lambda c: cof[c], 8 * lay.at["Z"])
+    return lay, consts, tables
+
+
+def kmt2_places(lay, name, P):
+    """The layout with a program's products and temporaries."""
+    at = dict(lay.at)
+    free = lay.place[name]
+    for op in P.ops:
+        for x in op[1:4]:
+            if isinstance(x, str) and x[0] in "pt":
+                if int(x[1:]) >= len(free):
+                    raise ValueError(f"{name}: too many temporaries")
+                at[x] = free[int(x[1:])]
+    return at
+
+
+def kmt2_sources() -> dict[str, str]:
+    lay, consts, tables = kmt2_tables()
+    text = (PKG / "csrc" / "gen" / "kmt2_aq.cuh").read_text()
+    body = re.search(r"void kq_add_diagonal\([^)]*\)\n\{\n(.*?)\n\}", text, re.S).group(1)
+    diag = [int(x) for x in re.findall(r"^\s*g\[(\d+) \* KQ_S\] =", body, re.M)]
+    rates = kmt2_rates()
+    banner = "// Generated by cmaq_gb300.mechgen.coop from gen/kmt2_aq.cuh.  Do not edit."
+    n = {k: -(-len(t) // CHUNK) for k, t in tables.items()}
+    first, pos = {}, 0
+    for k, v in n.items():
+        first[k], pos = pos, pos + v
+    order = ["fjac", "decomp", "solve", "solve", "fun", "solve", "fun", "solve"]
+    where, pos = "", 0                       # nested choice of the segment that chunk k of a pass lies in
+    for q, k in enumerate(order):
+        shift = first[k] - pos
+        pos += n[k]
+        where += (f"k < {pos} ? " if q < len(order) - 1 else "") + f"k + {shift}" + (" : " if q < len(order) - 1 else "")
+    dc, tc = _consts_text("c_kmt2_const", consts)
+    dr, tr = _rows_text("c_kmt2_rows", tables.values(), CHUNK)
+    cells = (SMEM_MAX - TABLE_SMEM - 8 * len(consts)) // (8 * lay.elems)
+    h = [banner, "// Sizes and tables of the cooperative KMT2 kernels (csrc/kmt2_coop.cuh).", "#pragma once",
+         "#include <cuda_runtime.h>", "namespace kmt2_coop {", dc, dr,
+         f"extern __device__ const short c_kmt2_diag[{len(diag)}];",
+         "struct Rate { int kind, r, i0, i1, i2; double p0, p1, p2; };   // 0 DISF, 1 DISB, 2 KRXN, 3 KIEPOX",
+         f"extern __device__ const Rate c_kmt2_rate[{len(rates)}];", "struct Coop {",
+         f"    static constexpr int ELEMS = {lay.elems}, NCONST = {len(consts)}, MAX_CELLS = {cells};",
+         f"    static constexpr int WS_ELEMS = {lay.ws_elems}, FACTOR = {lay.factor}, CELL = {lay.cell}, CELL_DOUBLES = 64, "
+         f"Z = {lay.at['Z']}, ONE = {lay.at['O']}, NRATE = {len(rates)};",
+         f"    static constexpr int CHUNK = {CHUNK}, TABLE_SMEM = {TABLE_SMEM};",
+         "    static constexpr int " + ", ".join(f"{k.upper()}_ROWS = {len(t)}" for k, t in tables.items()) + ";",
+         f"    // chunks of one pass ({', '.join(order)}), and where each lies",
+         f"    static constexpr int PASS = {pos};",
+         f"    static __device__ __forceinline__ int chunk(int k) {{ return {where}; }}",
+         "    static __device__ __forceinline__ const double* constants() { return c_kmt2_const; }",
+         "    static __device__ __forceinline__ const uint2* rows() { return c_kmt2_rows; }", "};",
+         "}  // namespace kmt2_coop"]
+    c = [banner, '#include "kmt2_coop_tables.cuh"', "namespace kmt2_coop {", tc, *tr,
+         f"__device__ const short c_kmt2_diag[{len(diag)}] = {{{', '.join(map(str, diag))}}};",
+         f"__device__ const Rate c_kmt2_rate[{len(rates)}] = {{",
+         *[f"  {{{k}, {r}, {', '.join(map(str, i))}, {', '.join(map(c_double, x))}}}," for k, r, i, x in rates], "};",
+         "}  // namespace kmt2_coop"]
+    return {"kmt2_coop_tables.cuh": "\n".join(h) + "\n", "kmt2_coop_tables.cu": "\n".join(c) + "\n"}
+
+
 def write(mech: str, out: Path | None = None) -> None:
     out = out or PKG / "csrc" / "gen"
     for name, text in sources(mech).items():
         (out / name).write_text(text)
 
 
+def write_kmt2(out: Path | None = None) -> None:
+    for name, text in kmt2_sources().items():
+        ((out or PKG / "csrc" / "gen") / name).write_text(text)
+
+
 if __name__ == "__main__":
+    write_kmt2()
     for mech_ in ("cb6r5_ae7_aq", "cracmm2"):
         write(mech_)

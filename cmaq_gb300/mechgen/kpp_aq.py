@@ -506,7 +506,6 @@ def device_consts(k: KppMech) -> str:
     """Sizes and species indices for the device code (``namespace kmt2``)."""
     out = ["// Generated by cmaq_gb300/mechgen/kpp_aq.py from CCTM/src/cloud/acm_ae7_kmt2 (KPP aqueous",
            "// mechanism of the KMT2 cloud chemistry).  Included inside namespace kmt2.  Do not edit.",
-           "#pragma once", "",
            f"constexpr int NVAR = {k.nvar};", f"constexpr int NFIX = {k.nfix};", f"constexpr int NREACT = {k.nreact};",
            f"constexpr int LU_NONZERO = {len(k.lu_irow)};", f"constexpr int NHENRY = {len(k.henry)};", ""]
     for name, i in sorted(k.index.items(), key=lambda t: t[1]):
@@ -548,8 +547,7 @@ def device_source(k: KppMech) -> str:
     out = ["// Generated by cmaq_gb300/mechgen/kpp_aq.py from CCTM/src/cloud/acm_ae7_kmt2: Henry's law",
            "// constants (aqchem_kmt.F90:371-396), rate constants (aqchem_Initialize.F90:491-636,",
            "// aqchem_Rates.F90:456-579), tolerances, Fun, Jac_SP, KppDecomp, KppSolve as straight-line",
-           "// code.  Included inside namespace kmt2 by csrc/kmt2.cuh.  Do not edit.",
-           "#pragma once", ""]
+           "// code.  Included inside namespace kmt2 by csrc/kmt2.cuh.  Do not edit.", ""]
     out.append("KQ_HD inline void kq_henry(Cell& c, float t2)\n{")
     for h, (name, kind, a, e) in enumerate(k.henry):
         if kind == "hlconst":
@@ -581,7 +579,9 @@ def device_source(k: KppMech) -> str:
     out.append("KQ_HD inline void kq_add_diagonal(double* g, double x)\n{")
     out += [f"    g[{d} * KQ_S] = g[{d} * KQ_S] + x;" for d in k.lu_diag[:-1]]
     out.append("}\n")
-    out.append(device_routines(k))
+    out.append("#if KMT2_STRIDE != 1   // with stride 1 they are the cooperative kernels' programs")
+    out.append(device_routines(k).rstrip("\n"))
+    out.append("#endif\n")
     return "\n".join(out)
 
 

@@ -34,6 +34,7 @@ int main(int argc, char** argv)
         if (mode == 2) y &= ~0xffffffffffull;
         if (mode == 3) x = (x & 0xfff0000000000000ull) | ((y + g() % 5 - 2) & 0xfffffffffffffull);
         if (mode == 4) { x &= ~0xffffffffffull; y |= 0xffffffull; }
+        if (mode == 5 && i % 64 == 5) x &= 0x8000000000000000ull;   // +-0 / b
         const double a = from(x), b = from(y);
         bool ok;
         const double q = fpdiv::quotient(a, b, &ok);

@@ -124,7 +124,19 @@ def test_gear_rows_carry_out_the_sequential_operations(mech):
         assert all(got[e] == want[e] for e in range(lay.elems) if e not in scratch), name
 
 
-@pytest.mark.parametrize("mech", ["cb6r5_ae7_aq", "cracmm2"])
+def test_kmt2_rows_carry_out_the_sequential_operations():
+    lay, consts, tables = C.kmt2_tables()
+    for name, prog in C.kmt2_programs().items():
+        at = C.kmt2_places(lay, name, prog)
+        ops = C.place(prog.ops, at)
+        term = Terms()
+        start = {e: term("in", e) for e in range(lay.elems)}
+        want, got = sequential(ops, start, term), rows_run(tables[name], start, consts, term)
+        scratch = {i for e, i in at.items() if e[0] in "pt"}
+        assert all(got[e] == want[e] for e in range(lay.elems) if e not in scratch), name
+
+
+@pytest.mark.parametrize("mech", ["cb6r5_ae7_aq", "cracmm2", "kmt2"])
 def test_tables_are_the_generated_ones(mech):
-    for name, text in C.sources(mech).items():
+    for name, text in (C.kmt2_sources() if mech == "kmt2" else C.sources(mech)).items():
         assert (C.PKG / "csrc" / "gen" / name).read_text() == text
