@@ -5,7 +5,7 @@
 // there are, because a lone warp issues one FP64 instruction per 64 cycles on GB300.  Here
 // the operations of an attempt (f, the iteration matrix and its factors, the solves) are
 // dealt out to the 32 lanes by a schedule made with the mechanism (mechgen/coop.py: rows of
-// one operation per lane, gen/<mech>_coop.cu), so an attempt of a CB6r5 cell takes 1,030 rows,
+// one operation per lane, gen/<mech>_coop.cu), so an attempt of a CB6r5 cell takes 1,440 rows,
 // and the state (25.8 KB, 8 cells per SM; CRACMM2 42.4 KB, 5) stays in shared memory.
 //
 // Measured (CB6r5): an attempt takes 212,000 cycles for one warp per SM and 285,000 for eight
@@ -309,8 +309,8 @@ __device__ __forceinline__ void run(S& st, int rows, uint32_t cell, uint32_t cst
 // One attempt of ros3::attempt_phased (rbsolver.F:344-589) on the warp's cell; the scalar state
 // is kept identically by the lanes.  Every warp of the block calls it; one with
 // active == false goes through the rows on whatever its cell holds.  yave: the cell's
-// time integral of Y in global memory (stride ystride), or nullptr.
-template <class M, class C>
+// time integral of Y in global memory (stride ystride), or nullptr.  ADJ: of the adjoint's forward pass.
+template <class M, class C, bool ADJ = false>
 __device__ __forceinline__ void attempt(double* __restrict__ x, Stream<C>& rows, uint32_t cst, ros3::CellState& s,
                                         double chemstep, ros3::Tol tol, int max_iter, bool active, double* yave,
                                         long long ystride)
@@ -411,7 +411,7 @@ __device__ __forceinline__ void attempt(double* __restrict__ x, Stream<C>& rows,
         }
     }
     if (accept) {
-        double dtfac = step_factor(maxerr);
+        double dtfac = step_factor<ADJ>(maxerr);
         s.st.nsteps++;
         if (bad) s.st.status |= ST_NONFINITE;
         s.tnow = tend;

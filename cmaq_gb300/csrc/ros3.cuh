@@ -60,10 +60,13 @@ __device__ __forceinline__ double fmax_keepnan(double a, double b) { return (b !
 // On the device: CUDA's pow is about 290 FP64 instructions, a quarter of what the lanes of the
 // cooperative kernel issue per attempt.  A cube root from the float exp2 / log2 (within 3e-6
 // where the factor is below FACMAX = 10, which clips it) and one third-order step is within
-// 1.5 ulp, as 0.9 / pow is.
+// 1.5 ulp, as 0.9 / pow is.  POW: by pow all the same, for the adjoint, whose gradients amplify a
+// step size's last bit (clipped and cancelling components by up to 2.5e-7 of the gradient).
+template <bool POW>
 __device__ __forceinline__ double step_factor(double maxerr)
 {
 #ifdef __CUDA_ARCH__
+    if (POW) return 0.9 / pow(maxerr, GROW);
     const double y0 = (double)exp2f(-__log2f((float)maxerr) * (1.0f / 3.0f));
     const double e = fma(-(maxerr * y0) * y0, y0, 1.0);
     return 0.9 * fma(y0 * e, fma(e, 2.0 / 9.0, 1.0 / 3.0), y0);
@@ -229,7 +232,7 @@ __device__ void attempt_phased(double* __restrict__ ws, CellState& s, double che
     }
     const double maxerr = fmax_keepnan(fmax(0.0, UROUND), sqrt(err * tol.rnspec));
     if (maxerr <= 1.0) {
-        double dtfac = step_factor(maxerr);
+        double dtfac = step_factor<EMIS>(maxerr);
         s.st.nsteps++;
         if (s.yave) {   // YAVE += (Y + Y') / 2 * DT (rbsolver.F:468-475)
             for (int n = 0; n < M::NSPEC; ++n) {
