@@ -100,6 +100,7 @@ struct cmaqchem_handle {
     int rconst_pass = 1;
     double* d_rki_all = nullptr;
     uint8_t* d_sun_all = nullptr;
+    int adj_coop = -1;       // cooperative adjoint kernels: -1 by size, 0 off, 1 always
     int coop = -1;           // cooperative ROS3 kernel: -1 by size (use_coop), 0 off, 1 always
     int q_sync = 1;          // work-queue kernel: barriers between attempt phases
     int q_wpb = 8;           // work-queue kernel: warps per block
@@ -476,6 +477,9 @@ extern "C" int cmaqchem_diag_set_tuning(cmaqchem_handle* h, const char* key, int
         if (h->graph_exec) CK(cudaGraphExecDestroy(h->graph_exec));
         h->graph_exec = nullptr;
         return 0;
+    } else if (strcmp(key, "adjoint_coop") == 0) {
+        if (value < -1 || value > 1) return fail("adjoint_coop must be -1 (by size), 0 or 1");
+        h->adj_coop = value;
     } else if (strcmp(key, "ros3_coop") == 0) {
         if (value < -1 || value > 1) return fail("ros3_coop must be -1 (by size), 0 or 1");
         h->coop = value;
@@ -977,18 +981,32 @@ int grow(T** p, size_t* cap, size_t need)
 
 int adj_setup(cmaqchem_handle* h, long long ncell)
 {
-    if (!h->d_adj_ws) {
-        int fb = 0, rb = 0;
-        CK(h->ops->adj_occupancy(&fb, &rb));
-        int bps = fb < rb ? fb : rb;
-        if (bps < 1) bps = 1;
-        h->adj_nblocks = h->nsm * bps;
-        CK(cudaMalloc(&h->d_adj_ws, (size_t)h->adj_nblocks * adj::WPB * h->ops->adj_ws_elems * 32 * sizeof(double)));
-        CK(cudaMalloc(&h->d_adj_counters, 3 * sizeof(unsigned long long)));
-    }
+    if (!h->d_adj_counters) CK(cudaMalloc(&h->d_adj_counters, 3 * sizeof(unsigned long long)));
     if (grow(&h->d_adj_order, &h->adj_cell_cap, (size_t)ncell)) return -1;
     if (grow(&h->d_adj_status, &h->adj_status_cap, (size_t)ncell)) return -1;
     return 0;
+}
+
+// The forward or reverse sweep of a queue of cells: cooperative up to the mechanism's limit,
+// above it one cell per lane (the same states, tapes and gradients of a cell), whose
+// workspaces are allocated by the first call that needs them.
+cudaError_t adj_launch(cmaqchem_handle* h, const adj::Args& a, bool reverse, cudaStream_t s)
+{
+    const long long n = a.queue_len > 0 ? a.queue_len : a.ncell;
+    if (h->adj_coop >= 0 ? h->adj_coop > 0 : n <= h->ops->adj_coop_limit) return h->ops->adj_coop(a, reverse, h->nsm, s);
+    if (!h->d_adj_ws) {
+        int fb = 0, rb = 0;
+        cudaError_t e = h->ops->adj_occupancy(&fb, &rb);
+        if (e != cudaSuccess) return e;
+        int bps = fb < rb ? fb : rb;
+        if (bps < 1) bps = 1;
+        h->adj_nblocks = h->nsm * bps;
+        e = cudaMalloc(&h->d_adj_ws, (size_t)h->adj_nblocks * adj::WPB * h->ops->adj_ws_elems * 32 * sizeof(double));
+        if (e != cudaSuccess) return e;
+    }
+    adj::Args b = a;
+    b.ws = h->d_adj_ws;
+    return reverse ? h->ops->adj_reverse(b, h->adj_nblocks, s) : h->ops->adj_forward(b, h->adj_nblocks, s);
 }
 
 // queue order of the cells by step counts, most first
@@ -1013,7 +1031,6 @@ adj::Args adj_args(cmaqchem_handle* h, long long ncell, const double* rki, const
     a.chemstep = chemstep;
     a.tol = ros3::Tol{h->cfg.rtol, h->cfg.atol, h->rnspec, h->dtmin};
     a.max_iter = h->max_iter;
-    a.ws = h->d_adj_ws;
     a.rki = rki;
     a.kmult = kmult;
     a.emis = emis;
@@ -1116,7 +1133,7 @@ extern "C" int cmaqchem_adj_forward(cmaqchem_handle* h, long long ncell, double*
             a.order = h->d_adj_order;
         }
         CK(cudaMemsetAsync(h->d_head, 0, sizeof(unsigned long long), s));
-        CK(h->ops->adj_forward(a, h->adj_nblocks, s));
+        CK(adj_launch(h, a, false, s));
     }
     unsigned long long cnt[3];
     CK(cudaMemcpyAsync(cnt, h->d_adj_counters, sizeof(cnt), cudaMemcpyDeviceToHost, s));
@@ -1161,7 +1178,7 @@ extern "C" int cmaqchem_adj_backward(cmaqchem_handle* h, long long ncell, double
             a.grad_logk = grad_logk;
             a.grad_emis = grad_emis;
             CK(cudaMemsetAsync(h->d_head, 0, sizeof(unsigned long long), s));
-            CK(h->ops->adj_reverse(a, h->adj_nblocks, s));
+            CK(adj_launch(h, a, true, s));
         }
         unsigned long long cnt[3];
         CK(cudaMemcpyAsync(cnt, h->d_adj_counters, sizeof(cnt), cudaMemcpyDeviceToHost, s));
@@ -1236,7 +1253,7 @@ extern "C" int cmaqchem_adj_backward(cmaqchem_handle* h, long long ncell, double
             a.grad_logk = grad_logk;
             a.grad_emis = grad_emis;
             CK(cudaMemsetAsync(h->d_head, 0, sizeof(unsigned long long), s));
-            CK(h->ops->adj_reverse(a, h->adj_nblocks, s));
+            CK(adj_launch(h, a, true, s));
             continue;
         }
         adj::Args a = adj_args(h, ncell, rki + (size_t)k * rki_sync_stride, night, kmult, emis, chemstep_min);
@@ -1284,13 +1301,13 @@ extern "C" int cmaqchem_adj_backward(cmaqchem_handle* h, long long ncell, double
             a.grad_logk = nullptr;
             a.grad_emis = nullptr;
             CK(cudaMemsetAsync(h->d_head, 0, sizeof(unsigned long long), s));
-            CK(h->ops->adj_forward(a, h->adj_nblocks, s));
+            CK(adj_launch(h, a, false, s));
             // reverse sweep
             a.lam = lambda;
             a.grad_logk = grad_logk;
             a.grad_emis = grad_emis;
             CK(cudaMemsetAsync(h->d_head, 0, sizeof(unsigned long long), s));
-            CK(h->ops->adj_reverse(a, h->adj_nblocks, s));
+            CK(adj_launch(h, a, true, s));
         }
     }
     unsigned long long cnt[3];

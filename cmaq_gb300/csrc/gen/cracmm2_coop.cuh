@@ -5,6 +5,8 @@
 namespace mech_cracmm2 {
 extern __device__ const double c_coop_const[544];
 extern __device__ const uint2 c_coop_rows[69888];
+extern __device__ const double c_coopadj_const[544];
+extern __device__ const uint2 c_coopadj_rows[120064];
 extern __device__ const double c_coopebi_const[550];
 extern __device__ const uint2 c_coopebi_rows[13440];
 extern __device__ const double c_coopgear_const[544];
@@ -19,6 +21,22 @@ struct Coop {
     static __device__ __forceinline__ int chunk(int k) { return k < 78 ? k : k - 15; }
     static __device__ __forceinline__ const double* constants() { return c_coop_const; }
     static __device__ __forceinline__ const uint2* rows() { return c_coop_rows; }
+};
+struct CoopAdj {
+    static constexpr int ELEMS = 6958, NCONST = 544, MAX_CELLS = 3;
+    static constexpr int Y = 0, V = 189, K1 = 378, K2 = 567, T = 756, K3 = 945, NU2 = 1134, NU3 = 1323, PHI = 1512, LAM = 1701, EMIS = 1890, RKI = 2079, GK = 3141, G = 6956, Z = 6957;
+    static constexpr int CHUNK = 28, TABLE_SMEM = 15936;
+    static constexpr int STAGE1_ROWS = 1408, RHS_ROWS = 324, SOLVE_ROWS = 420, TSOLVE_ROWS = 684, JTV_ROWS = 180, GRADIENT_ROWS = 652;
+    // chunks of one pass through the programs (stage1, rhs, solve, solve, tsolve, tsolve, jtv, tsolve, gradient), and where each lies
+    static constexpr int PASS = 199;
+    static __device__ __forceinline__ int chunk(int k) { return k < 78 ? k : k < 118 ? k - 15 : k < 150 ? k - 40 : k < 175 ? k - 72 : k - 65; }
+    static __device__ __forceinline__ const double* constants() { return c_coopadj_const; }
+    static __device__ __forceinline__ const uint2* rows() { return c_coopadj_rows; }
+};
+// the forward pass's programs of the same tables: stage1, rhs, solve, solve
+struct CoopAdjForward : CoopAdj {
+    static constexpr int PASS = 93;
+    static __device__ __forceinline__ int chunk(int k) { return k < 78 ? k : k - 15; }
 };
 struct CoopEbi {
     static constexpr int ELEMS = 3067, NCONST = 550, MAX_CELLS = 8;

@@ -9,6 +9,10 @@ namespace mech_cb6r5_ae7_aq {
 // 36,000 cells take 202 ms there and 271 ms one cell per lane, 126,000 cells 707 and 386 ms; a
 // later call of the hour 30 and 53 ms, 104 and 81 ms.
 constexpr long long COOP_LIMIT = 60000;
+// Adjoint windows of at most this many cells take the cooperative kernels: two steps and their
+// reverse take 221 ms there and 1,102 ms one cell per lane for 8,000 cells, 1,296 and 1,591 ms for
+// 50,000, 1,553 and 1,582 ms for 60,000, 2,062 and 1,716 ms for 80,000.
+constexpr long long ADJ_COOP_LIMIT = 55000;
 }
 
 DEFINE_MECH_OPS(mech_cb6r5_ae7_aq, mech_ops_cb6r5_ae7_aq)

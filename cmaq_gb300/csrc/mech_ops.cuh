@@ -9,6 +9,7 @@
 #include "adjoint.cuh"
 #include "ddm.cuh"
 #include "gear.cuh"
+#include "adj_coop.cuh"
 #include "coop.cuh"
 #include "ebi_coop.cuh"
 #include "gear_coop.cuh"
@@ -62,6 +63,9 @@ struct MechOps {
     int coop_max_cells;
     long long coop_limit;
     cudaError_t (*chem_coop)(const chem::GridArgs&, const chem::QueueArgs&, int cells, int nblocks, cudaStream_t);
+    // cooperative adjoint kernels, taken for at most adj_coop_limit cells
+    long long adj_coop_limit;
+    cudaError_t (*adj_coop)(const adj::Args&, bool reverse, int nsm, cudaStream_t);
 };
 
 #define DEFINE_MECH_OPS(NS, SYMBOL)                                                                 \
@@ -151,6 +155,22 @@ struct MechOps {
     cudaError_t adj_reverse_(const adj::Args& a, int nb, cudaStream_t s)                            \
     {                                                                                               \
         adj::k_adj_reverse<T_><<<nb, adj::THREADS, 0, s>>>(a);                                      \
+        return cudaGetLastError();                                                                  \
+    }                                                                                               \
+    cudaError_t adj_coop_(const adj::Args& a, bool reverse, int nsm, cudaStream_t s)                \
+    {                                                                                               \
+        using F = NS::CoopAdjForward;                                                               \
+        using R = NS::CoopAdj;                                                                      \
+        const long long n = a.queue_len > 0 ? a.queue_len : a.ncell;                                \
+        const int cells = (int)std::min<long long>(R::MAX_CELLS, (n + nsm - 1) / nsm);              \
+        const int nb = (int)std::min<long long>(nsm, (n + cells - 1) / cells);                      \
+        const size_t bytes = coop::smem_bytes<R>(cells);                                            \
+        const void* f = reverse ? (const void*)coop::k_adj_reverse_coop<T_, R>                      \
+                                : (const void*)coop::k_adj_forward_coop<T_, F>;                     \
+        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); \
+        if (e != cudaSuccess) return e;                                                             \
+        if (reverse) coop::k_adj_reverse_coop<T_, R><<<nb, cells * 32, bytes, s>>>(a);              \
+        else coop::k_adj_forward_coop<T_, F><<<nb, cells * 32, bytes, s>>>(a);                      \
         return cudaGetLastError();                                                                  \
     }                                                                                               \
     cudaError_t adj_occupancy_(int* f, int* r)                                                      \
@@ -252,4 +272,5 @@ struct MechOps {
                                    T_::EBI_DELTAT,                                                  \
                                    T_::ADJ_WS_ELEMS, adj_forward_, adj_reverse_, adj_occupancy_, ddm_update_,     \
                                    rconst_, rconst_pass_, occupancy_, T_::GEAR_WS_ELEMS, gear_, gear_occupancy_, \
-                                   gear_warp_, gear_warp_occupancy_, NS::Coop::MAX_CELLS, NS::COOP_LIMIT, chem_coop_};
+                                   gear_warp_, gear_warp_occupancy_, NS::Coop::MAX_CELLS, NS::COOP_LIMIT, chem_coop_, \
+                                   NS::ADJ_COOP_LIMIT, adj_coop_};

@@ -427,6 +427,180 @@ def ros3_tables(mech: str, width: int = WIDTH):
     return lay, consts, tables
 
 
+# ----------------------------------------------------------------------------- discrete adjoint of ROS3
+
+def transposed_substitution(P: Program, sp, v: str):
+    """A^T x = b in place, U^T by ascending rows, then L^T by descending ones (emit_cuda._solve_t_chunks)."""
+    n = sp.ischan
+    col_u, col_l = [[] for _ in range(n)], [[] for _ in range(n)]
+    for k in range(n):
+        for st, j in sp.upper[0][k]:
+            col_u[j].append((k, st))
+        for st, j in sp.lower[0][k]:
+            col_l[j].append((k, st))
+    for i in range(n):
+        for k, st in sorted(col_u[i]):
+            P.fma(f"{v}{i}", f"A{st}", f"{v}{k}", neg=True)
+        P.fma(f"{v}{i}", f"{v}{i}", f"A{sp.jarraypt[0][(i, i)]}", init=NEG0)
+    for i in range(n - 1, -1, -1):
+        for k, st in sorted(col_l[i]):
+            P.fma(f"{v}{i}", f"A{st}", f"{v}{k}", neg=True)
+
+
+def stoich_sum(P: Program, m, sp, r: int, vec: str, d: str):
+    """d = reaction r's net stoichiometry times vec (emit_cuda._stoich_sum)."""
+    for p in range(m.nprdct[r]):
+        P.fma(d, f"{vec}{sp.irm2[r][3 + p]}", ("c", m.sc[r][p]), init=NEG0 if p == 0 else LOAD)
+    for i in range(m.nreact[r]):
+        P.fma(d, f"{vec}{sp.irm2[r][i]}", ("c", 1.0), neg=True, init=NEG0 if not m.nprdct[r] and i == 0 else LOAD)
+
+
+def jtv(P: Program, m, sp, y: str, out: str, temp):
+    """out += J(y)^T P and W_r += w_r R_r(y) (emit_cuda._adj_jtv); w_r and then RKI_r w_r in X_r."""
+    for r in sp.active[0]:
+        nre = m.nreact[r]
+        if nre == 0 and m.nprdct[r] == 0:
+            continue
+        stoich_sum(P, m, sp, r, "P", f"X{r}")
+        P.fma(f"X{r}", f"X{r}", f"R{r}", init=NEG0)
+        a = [sp.irm2[r][i] for i in range(nre)]
+        if nre == 0:
+            P.fma(f"W{r}", f"X{r}", ("c", 1.0))
+        elif nre == 1:
+            P.fma(f"{out}{a[0]}", f"X{r}", ("c", 1.0))
+            P.fma(f"W{r}", f"X{r}", f"{y}{a[0]}")
+        elif nre == 2:
+            P.fma(f"{out}{a[0]}", f"X{r}", f"{y}{a[1]}")
+            P.fma(f"{out}{a[1]}", f"X{r}", f"{y}{a[0]}")
+            P.fma(f"X{r}", f"X{r}", f"{y}{a[0]}", init=NEG0)
+            P.fma(f"W{r}", f"X{r}", f"{y}{a[1]}")
+        else:
+            t = temp()
+            P.fma(t, f"X{r}", f"{y}{a[1]}", init=NEG0)
+            P.fma(f"{out}{a[0]}", t, f"{y}{a[2]}")
+            P.fma(f"X{r}", f"X{r}", f"{y}{a[0]}", init=NEG0)
+            P.fma(f"{out}{a[1]}", f"X{r}", f"{y}{a[2]}")
+            P.fma(f"{out}{a[2]}", f"X{r}", f"{y}{a[1]}")
+            P.fma(f"X{r}", f"X{r}", f"{y}{a[1]}", init=NEG0)
+            P.fma(f"W{r}", f"X{r}", f"{y}{a[2]}")
+
+
+def hess3(P: Program, m, sp, temp):
+    """The stage solves' second-order terms (emit_cuda._adj_hess3): nu in V, C, D, the stages in K, L, Q."""
+    for r in sp.active[0]:
+        nre = m.nreact[r]
+        if nre == 0:
+            continue
+        a = [sp.irm2[r][i] for i in range(nre)]
+        w = [temp() for _ in range(3)]
+        for v, x in zip("VCD", w):
+            stoich_sum(P, m, sp, r, v, x)
+        wk = []
+        for s in a:
+            wk.append(temp())
+            for v, x, init in zip("KLQ", w, (NEG0, LOAD, LOAD)):
+                P.fma(wk[-1], x, f"{v}{s}", init=init)
+        y = [f"Y{s}" for s in a]
+
+        def pair(u, i, v, j):        # u * wk_i + v * wk_j
+            t = temp()
+            P.fma(t, v, wk[j], init=NEG0)
+            P.fma(t, u, wk[i])
+            return t
+        if nre == 1:
+            P.fma(f"W{r}", f"R{r}", wk[0], neg=True)
+        elif nre == 2:
+            P.fma(f"W{r}", f"R{r}", pair(y[1], 0, y[0], 1), neg=True)
+            P.fma(f"M{a[0]}", f"R{r}", wk[1], neg=True)
+            P.fma(f"M{a[1]}", f"R{r}", wk[0], neg=True)
+        else:
+            t = temp()
+            P.fma(t, y[0], y[1], init=NEG0)
+            P.fma(t, t, wk[2], init=NEG0)
+            for u, v, k in ((0, 2, 1), (1, 2, 0)):
+                q = temp()
+                P.fma(q, y[u], y[v], init=NEG0)
+                P.fma(t, q, wk[k])
+            P.fma(f"W{r}", f"R{r}", t, neg=True)
+            P.fma(f"M{a[0]}", f"R{r}", pair(y[2], 1, y[1], 2), neg=True)
+            P.fma(f"M{a[1]}", f"R{r}", pair(y[2], 0, y[0], 2), neg=True)
+            P.fma(f"M{a[2]}", f"R{r}", pair(y[1], 0, y[0], 1), neg=True)
+
+
+def adjoint_programs(m, sp) -> tuple[dict[str, Program], list, list]:
+    """Of the step and its adjoint (csrc/adj_coop.cuh): stage1, rhs and solve as ros3_programs' with the
+    emission tendency N added to f, tsolve (V), jtv (V += J(T)^T P) and gradient (M += J(Y)^T P, then
+    the second-order terms).  Returns also the temporaries of jtv and of gradient."""
+    p = {k: Program() for k in ("stage1", "rhs", "solve", "tsolve", "jtv", "gradient")}
+    for name, src, dst in (("stage1", "Y", "V"), ("rhs", "T", "T")):
+        rates(p[name], m, sp, src)
+        tendency(p[name], m, sp, dst)
+        for i in range(sp.ischan):
+            p[name].fma(f"{dst}{i}", f"N{i}", ("c", 1.0))
+    partials(p["stage1"], m, sp)
+    iteration_matrix(p["stage1"], m, sp)
+    substitution(p["stage1"], m, sp, "V")
+    substitution(p["solve"], m, sp, "V")
+    transposed_substitution(p["tsolve"], sp, "V")
+    temps = {"j": [], "h": []}
+
+    def temp(kind):
+        temps[kind].append(f"{kind}{len(temps[kind])}")
+        return temps[kind][-1]
+    jtv(p["jtv"], m, sp, "T", "V", lambda: temp("j"))
+    jtv(p["gradient"], m, sp, "Y", "M", lambda: temp("h"))
+    hess3(p["gradient"], m, sp, lambda: temp("h"))
+    return p, temps["j"], temps["h"]
+
+
+class AdjointLayout:
+    """Element offsets (doubles) of a cell's state.  The partial-derivative products lie over vectors that
+    are formed after the factors; the gradient's temporaries over the factors, in turn."""
+
+    VECTORS = dict(y="Y", v="V", k1="K", k2="L", t="T", k3="Q", nu2="C", nu3="D", phi="P", lam="M", emis="N")
+
+    def __init__(self, m, sp, jtemps, htemps):
+        n, nr = m.nspec, m.nrxns
+        self.at, off = {}, 0
+        for name, v in self.VECTORS.items():
+            self.at.update({f"{v}{i}": off + i for i in range(n)})
+            setattr(self, name, off)
+            off += n
+        for name, v in (("rki", "R"), ("x", "X"), ("gk", "W")):
+            self.at.update({f"{v}{r}": off + r for r in range(nr)})
+            setattr(self, name, off)
+            off += nr
+        self.lu = off
+        self.at.update({f"A{st}": off + st - 1 for st in range(1, sp.iarray[0] + 1)})
+        off += sp.iarray[0]
+        self.g, self.z = off, off + 1
+        self.at.update(G=off, Z=off + 1)
+        off += 2
+        self.at.update({e: off + q for q, e in enumerate(jtemps)})
+        self.elems = off + len(jtemps)
+        ex = [f"E{r}_{q}" for r in sp.active[0] if m.nreact[r] >= 2 for q in range(m.nreact[r])]
+        if len(ex) > 7 * n:
+            raise ValueError("no room for the partial-derivative products")
+        self.at.update({e: self.k1 + q for q, e in enumerate(ex)})          # K1 ... PHI
+        self.at.update({e: self.lu + q % sp.iarray[0] for q, e in enumerate(htemps)})
+        if 8 * self.elems > 1 << 16:
+            raise ValueError("an operation's offsets have 16 bits")
+
+
+def adjoint_tables(mech: str, width: int = WIDTH):
+    """(layout, constants, {program: encoded rows})."""
+    m, sp = mechanism(mech)
+    progs, jtemps, htemps = adjoint_programs(m, sp)
+    lay = AdjointLayout(m, sp, jtemps, htemps)
+    consts = sorted({op[3][1] for p in progs.values() for op in p.ops if isinstance(op[3], tuple)})
+    cof = {c: 8 * q for q, c in enumerate(consts)}
+    tables = {}
+    for name, p in progs.items():
+        ops = place(p.ops, lay.at)
+        tables[name] = encode(ops, schedule(ops, width), lambda e: 8 * e, lambda c: cof[c], 8 * lay.z)
+    return lay, consts, tables
+
+
 class GearLayout:
     """Places of SMVGEAR's programs in the one-cell workspace of the Gear kernels (emit_cuda.Layout):
     a pivot's reciprocal takes the pivot's place, the concentrations with CEFF's zeros the place of
@@ -807,6 +981,17 @@ def _consts_text(sym, consts):
             f"__device__ const double {sym}[{len(consts)}] = {{{', '.join(map(c_double, consts))}}};")
 
 
+def reverse_chunk(n: dict) -> str:
+    """Where chunk k of the reverse step's pass lies: its second solve and second and third tsolve
+    are the first ones' chunks again."""
+    s = n["stage1"] + n["rhs"] + n["solve"]            # end of the first solve
+    t = s + n["solve"] + n["tsolve"]                   # of the first tsolve
+    j = t + n["tsolve"] + n["jtv"]                     # of jtv
+    again = n["solve"] + n["tsolve"]
+    return (f"k < {s} ? k : k < {t} ? k - {n['solve']} : k < {j} ? k - {again} : "
+            f"k < {j + n['tsolve']} ? k - {again + n['tsolve'] + n['jtv']} : k - {again + n['tsolve']}")
+
+
 def sources(mech: str) -> dict[str, str]:
     """<mech>_coop.cuh (sizes) and <mech>_coop.cu (tables)."""
     banner = [f"// Generated by cmaq_gb300.mechgen.coop from mechs/{mech}/manifest.json and gen/{mech}_ebi.cu.  Do not edit."]
@@ -838,6 +1023,16 @@ def sources(mech: str) -> dict[str, str]:
                   dict(Y=lay.y, V=lay.v, K1=lay.k, K2=lay.l, T=lay.t, RKI=lay.rki, G=lay.g, Z=lay.z),
                   ["stage1", "rhs", "solve", "solve"],
                   lambda n: f"k < {sum(n.values())} ? k : k - {n['solve']}")
+    alay, aconsts, atabs = adjoint_tables(mech)
+    tail += traits("CoopAdj", alay, aconsts, atabs,
+                   dict(Y=alay.y, V=alay.v, K1=alay.k1, K2=alay.k2, T=alay.t, K3=alay.k3, NU2=alay.nu2, NU3=alay.nu3,
+                        PHI=alay.phi, LAM=alay.lam, EMIS=alay.emis, RKI=alay.rki, GK=alay.gk, G=alay.g, Z=alay.z),
+                   ["stage1", "rhs", "solve", "solve", "tsolve", "tsolve", "jtv", "tsolve", "gradient"], reverse_chunk)
+    step = [-(-len(atabs[k]) // CHUNK) for k in ("stage1", "rhs", "solve")]
+    tail += ["// the forward pass's programs of the same tables: stage1, rhs, solve, solve",
+             "struct CoopAdjForward : CoopAdj {",
+             f"    static constexpr int PASS = {sum(step) + step[2]};",
+             f"    static __device__ __forceinline__ int chunk(int k) {{ return k < {sum(step)} ? k : k - {step[2]}; }}", "};"]
     elay, econsts, rows = ebi_tables(mech)
     tail += traits("CoopEbi", elay, econsts, {"iteration": rows},
                    dict(YC=elay.yc, YC0=elay.yc0, YCP=elay.ycp, PROD=elay.prod, LOSS=elay.loss, PNEG=elay.pneg,

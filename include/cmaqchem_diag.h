@@ -54,6 +54,9 @@ int cmaqchem_diag_fp64_issue(int device, int active_lanes, double* cycles_per_in
  * "ros3_coop" (ROS3: 1 the cooperative kernel, one cell per warp with its state in shared
  * memory, where the rate-constant pass's arrays were allocated, 0 one cell per lane, -1
  * (default) by the size of the call; same results) and
+ * "adjoint_coop" (the adjoint's passes: 1 one cell per warp with its state in shared memory, 0 one
+ * cell per lane, -1 (default) by the number of cells; the same states and gradients of a cell,
+ * the rate gradients summed over the cells in another order) and
  * "queue_history" (0: clear the step counts the work queue is ordered by, so that the next
  * call is queued as a fresh run's first call; synchronises the device before and after) and
  * "host_chunks" (1-16, default 4: cmaqchem_step moves the grid in that many chunks of

@@ -124,6 +124,27 @@ def test_gear_rows_carry_out_the_sequential_operations(mech):
         assert all(got[e] == want[e] for e in range(lay.elems) if e not in scratch), name
 
 
+@pytest.mark.parametrize("mech", ["cb6r5_ae7_aq", "cracmm2"])
+def test_adjoint_rows_carry_out_the_sequential_operations(mech):
+    m, sp = C.mechanism(mech)
+    lay, consts, tables = C.adjoint_tables(mech)
+    for name, prog in C.adjoint_programs(m, sp)[0].items():
+        ops = C.place(prog.ops, lay.at)
+        term = Terms()
+        start = {e: term("in", e) for e in range(lay.elems)}
+        want, got = sequential(ops, start, term), rows_run(tables[name], start, consts, term)
+        # products of the matrix (E) and the gradient's temporaries (h) are scratch
+        scratch = {i for e, i in lay.at.items() if e[0] in {"stage1": "E", "gradient": "h"}.get(name, "")}
+        assert all(got[e] == want[e] for e in range(lay.elems) if e not in scratch), name
+    n = {k: -(-len(t) // C.CHUNK) for k, t in tables.items()}
+    first = dict(zip(n, [sum(list(n.values())[:i]) for i in range(len(n))]))
+    order = ["stage1", "rhs", "solve", "solve", "tsolve", "tsolve", "jtv", "tsolve", "gradient"]
+    chunk = C.reverse_chunk(n).replace("?", "and").replace(":", "or")
+    for k, want in enumerate(first[p] + i for p in order for i in range(n[p])):
+        # Python's `c and a or b` is C's `c ? a : b` but for a == 0, which is chunk 0's
+        assert eval(chunk, {"k": k}) == want or k == want == 0
+
+
 def test_kmt2_rows_carry_out_the_sequential_operations():
     lay, consts, tables = C.kmt2_tables()
     for name, prog in C.kmt2_programs().items():

@@ -112,3 +112,39 @@ def test_gear_cells_that_reach_the_evaluation_cap():
     s.set_tuning(gear_warp=0)
     assert 0 < a[1][0]["failed_cells"] < 90
     same(run(s, t, -1, 1), a)
+
+
+def gradients(s, t, nsync, mode, tape_bytes=None):
+    import torch
+    from cmaq_gb300.adjoint import Ros3Window
+    s.set_tuning(adjoint_coop=mode)
+    w = Ros3Window(s, t["rki"], t["night"], nsync, 5.0, tape_bytes=tape_bytes)
+    x = [t[k].clone().requires_grad_(True) for k in ("y0", "log_k", "emis")]
+    y = w(*x)
+    g = torch.autograd.grad(y, x, t["cost"])
+    return [v.detach().cpu().numpy() for v in (y, g[0], g[2], g[1])]
+
+
+@pytest.mark.parametrize("mech,cells,tape,tape_mb", [("cb6r5_ae7_aq", 1, None, 0), ("cb6r5_ae7_aq", 913, None, 0),
+                                                     ("cb6r5_ae7_aq", 150, 0, 0), ("cb6r5_ae7_aq", 150, 0, 1),
+                                                     ("cracmm2", 457, None, 0)])
+def test_adjoint_as_one_cell_per_lane(mech, cells, tape, tape_mb):
+    """States and the gradients of a cell bit for bit, with the tape recorded by the forward pass, re-run whole,
+    and in batches; the rate gradients, sums over the cells in another order, within 100 roundings of the
+    sum of the terms' magnitudes, which the largest gradient stands for up to their cancellation (1e-10)."""
+    import torch
+    from helpers import gather_cells
+    from oracle import Oracle
+    from cmaq_gb300.chem import ChemSolver
+    g = make_grid(mech=mech, ncols=cells, nrows=1, nlays=1, seed=51, het=True)
+    y0, rki, night = gather_cells(g, Oracle(mech))
+    rng = np.random.default_rng(7)
+    t = {k: torch.from_numpy(np.ascontiguousarray(v)).cuda() for k, v in dict(
+        y0=y0, rki=rki, night=night, log_k=0.05 * rng.standard_normal(rki.shape[0]), emis=1e-6 * rng.random(y0.shape),
+        cost=rng.standard_normal(y0.shape) / np.maximum(y0, 1e-12)).items()}
+    s = ChemSolver(mech, ncols=cells, nrows=1, nlays=1, nspcsd=g.nspcsd, rtol=1e-3, atol=1e-9)
+    s.set_tuning(adjoint_tape_mb=tape_mb)
+    a, b = gradients(s, t, 2, 1, tape), gradients(s, t, 2, 0, tape)
+    for u, v in zip(a[:3], b[:3]):
+        assert np.array_equal(u, v)
+    assert np.max(np.abs(a[3] - b[3])) <= 1e-10 * np.max(np.abs(b[3]))
