@@ -102,6 +102,9 @@ struct cmaqchem_handle {
     uint8_t* d_sun_all = nullptr;
     int adj_coop = -1;       // cooperative adjoint kernels: -1 by size, 0 off, 1 always
     int coop = -1;           // cooperative ROS3 kernel: -1 by size (use_coop), 0 off, 1 always
+    int hand_over = -1;      // work-queue kernel: what a block hands over at most, -1: 3/8 of its lanes
+    chem::HandOver d_over{}; // room for the cells of every block
+    size_t over_cap = 0;
     int q_sync = 1;          // work-queue kernel: barriers between attempt phases
     int q_wpb = 8;           // work-queue kernel: warps per block
     int q_nblocks = 0;
@@ -166,7 +169,8 @@ void free_handle(cmaqchem_handle* h)
                     h->s_qv, h->s_dens, h->s_pres, h->s_seaice, h->s_osz, h->s_rj, h->s_khet,
                     h->d_adj_ws, h->d_tape_y, h->d_tape_h, h->d_tape_off, h->d_tiles, h->d_tape_tot,
                     h->d_adj_order, h->d_adj_status, h->d_adj_counters, h->d_yave, h->d_gear_coef,
-                    h->d_ebi_def, h->d_ebi_ndef, h->d_rki_all, h->d_sun_all};
+                    h->d_ebi_def, h->d_ebi_ndef, h->d_rki_all, h->d_sun_all, h->d_over.count, h->d_over.cell,
+                    h->d_over.slot, h->d_over.state};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
@@ -213,7 +217,24 @@ int configure_queue(cmaqchem_handle* h)
     if (bps < 1) bps = 1;
     if (h->q_bps_cap > 0 && bps > h->q_bps_cap) bps = h->q_bps_cap;
     h->q_nblocks = h->nsm * bps;
-    return ensure_ws(h, (size_t)h->q_nblocks * h->q_wpb);
+    if (ensure_ws(h, (size_t)h->q_nblocks * h->q_wpb)) return -1;
+    const size_t lanes = (size_t)h->q_nblocks * h->q_wpb * 32;
+    if (lanes > h->over_cap) {
+        void* ptrs[] = {h->d_over.count, h->d_over.cell, h->d_over.slot, h->d_over.state};
+        for (void* p : ptrs)
+            if (p) CK(cudaFree(p));
+        h->d_over = chem::HandOver{};
+        h->over_cap = 0;
+        if (cudaMalloc(&h->d_over.count, sizeof(unsigned long long)) == cudaSuccess &&
+            cudaMalloc(&h->d_over.cell, sizeof(long long) * lanes) == cudaSuccess &&
+            cudaMalloc(&h->d_over.slot, sizeof(int) * lanes) == cudaSuccess &&
+            cudaMalloc(&h->d_over.state, sizeof(ros3::CellState) * lanes) == cudaSuccess) {
+            h->over_cap = lanes;
+        } else {
+            cudaGetLastError();   // no room: the kernel finishes all of its cells itself
+        }
+    }
+    return 0;
 }
 
 // Whether a ROS3 call of n cells takes the cooperative kernel (same results): below the
@@ -480,6 +501,9 @@ extern "C" int cmaqchem_diag_set_tuning(cmaqchem_handle* h, const char* key, int
     } else if (strcmp(key, "adjoint_coop") == 0) {
         if (value < -1 || value > 1) return fail("adjoint_coop must be -1 (by size), 0 or 1");
         h->adj_coop = value;
+    } else if (strcmp(key, "ros3_hand_over") == 0) {
+        if (value < -1) return fail("ros3_hand_over must be >= -1");
+        h->hand_over = value;
     } else if (strcmp(key, "ros3_coop") == 0) {
         if (value < -1 || value > 1) return fail("ros3_coop must be -1 (by size), 0 or 1");
         h->coop = value;
@@ -619,7 +643,24 @@ static int enqueue_step(cmaqchem_handle* h, const chem::GridArgs& a, int itmstep
                 const int nb = (int)std::min<long long>(h->nsm, (n + cells - 1) / cells);
                 CK(h->ops->chem_coop(ap, q, cells, nb, s));
             } else {
+                // Once a block has at most 3/8 of its lanes left it hands its cells over to the cooperative
+                // kernel: the first, second and third call of 126,000 CB6r5 cells take 362 / 68 / 56 ms, with
+                // a quarter 378 / 69 / 56, half 363 / 69 / 56, three quarters 388 / 70 / 57, and without it
+                // 570 / 116 / 84; 360,000 cells 800 / 157 / 125 (996 / 192 / 142 without), 60,000 CRACMM2
+                // cells 789 / 171 / 161 (1,052 / 561 / 479).
+                const int lanes = h->q_wpb * 32;
+                const int most = h->q_sync == 0 || h->over_cap == 0 ? 0
+                               : h->hand_over >= 0 ? std::min(h->hand_over, lanes - 1) : lanes * 3 / 8;
+                if (most > 0) {
+                    q.over = h->d_over;
+                    q.over.most = most;
+                    CK(cudaMemsetAsync(h->d_over.count, 0, sizeof(unsigned long long), s));
+                }
                 CK(h->ops->chem_queue(ap, q, h->q_sync, h->q_wpb, h->q_nblocks, s));
+                if (most > 0) {
+                    CK(cudaMemsetAsync(h->d_head, 0, sizeof(unsigned long long), s));
+                    CK(h->ops->chem_coop(ap, q, h->ops->coop_max_cells, h->nsm, s));
+                }
             }
         } else {
             CK(h->ops->chem_queue(a, q, h->q_sync, h->q_wpb, h->q_nblocks, s));

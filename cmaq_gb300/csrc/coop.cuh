@@ -443,7 +443,8 @@ __global__ void __launch_bounds__(C::MAX_CELLS * 32, 1) k_chem_ros3_coop(chem::G
     for (int i = sub; i < C::ELEMS; i += W) x[i] = 0.0;
     Stream<C> rows;
     rows.start(coop_smem);
-    const unsigned long long qlen = chem::queue_len(q, a.ncell);
+    const bool unfinished = q.over.count != nullptr;   // goes on with the cells that were handed over
+    const unsigned long long qlen = unfinished ? *q.over.count : chem::queue_len(q, a.ncell);
     ros3::CellState s;
     ros3::start(s);
     long long cell = -1;
@@ -455,7 +456,17 @@ __global__ void __launch_bounds__(C::MAX_CELLS * 32, 1) k_chem_ros3_coop(chem::G
             unsigned long long pos = 0;
             if (need && sub == 0) pos = atomicAdd(q.head, 1ull);
             pos = __shfl_sync(0xffffffffu, pos, 0);
-            if (need && pos < qlen) {
+            if (need && pos < qlen && unfinished) {
+                cell = q.over.cell[pos];
+                const int slot = q.over.slot[pos];
+                const double* ws = a.ws + (size_t)(slot >> 5) * ((size_t)M::WS_ELEMS * 32) + (slot & 31);
+                for (int i = sub; i < M::ISCHAN; i += W) x[C::Y + i] = ws[(M::OFF_Y + i) * 32];
+                for (int r = sub; r < M::NRXNS; r += W) x[C::RKI + r] = a.rki_all[(size_t)r * a.ncell + cell];
+                if (a.yave)
+                    for (int i = sub; i < M::ISCHAN; i += W) a.yave[(size_t)i * a.ncell + cell] = ws[(M::OFF_YAVE + i) * 32];
+                sun = a.sun_all[cell] != 0;
+                s = q.over.state[pos];
+            } else if (need && pos < qlen) {
                 cell = q.cell0 + (q.order ? q.order[pos] : (long long)pos);
                 const float svol = __fdiv_rn(1.0f, a.dens[cell]);
                 for (int i = sub; i < M::ISCHAN; i += W) {   // as gather_cell_pass

@@ -5,10 +5,10 @@
 #include "mech_ops.cuh"
 
 namespace mech_cb6r5_ae7_aq {
-// Calls of at most this many cells take the cooperative ROS3 kernel: from the initial state
-// 36,000 cells take 202 ms there and 271 ms one cell per lane, 126,000 cells 707 and 386 ms; a
-// later call of the hour 30 and 53 ms, 104 and 81 ms.
-constexpr long long COOP_LIMIT = 60000;
+// Calls of at most this many cells take the cooperative ROS3 kernel, larger ones the work queue,
+// which hands its last cells over to it: the first, second and third call of 36,000 cells take 182 /
+// 36 / 29 ms there and 197 / 48 / 35 ms by the queue, of 54,000 cells 270 / 54 / 43 and 265 / 52 / 42.
+constexpr long long COOP_LIMIT = 50000;
 // Adjoint windows of at most this many cells take the cooperative kernels: two steps and their
 // reverse take 221 ms there and 1,102 ms one cell per lane for 8,000 cells, 1,296 and 1,591 ms for
 // 50,000, 1,553 and 1,582 ms for 60,000, 2,062 and 1,716 ms for 80,000.

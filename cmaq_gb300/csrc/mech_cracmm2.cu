@@ -5,10 +5,11 @@
 #include "mech_ops.cuh"
 
 namespace mech_cracmm2 {
-// Calls of at most this many cells take the cooperative ROS3 kernel: from the initial state
-// 10,881 cells take 267 ms there and 701 ms one cell per lane, 50,000 cells 1,190 and 962 ms; a
-// later call of the hour 26 and 232 ms, 116 and 282 ms.
-constexpr long long COOP_LIMIT = 40000;
+// Calls of at most this many cells take the cooperative ROS3 kernel, larger ones the work queue,
+// which hands its last cells over to it: the first, second and third call of 20,000 cells take 449 /
+// 81 / 56 ms there and 559 / 100 / 115 ms by the queue, of 40,000 cells 877 / 148 / 99 and 673 /
+// 134 / 120.
+constexpr long long COOP_LIMIT = 27000;
 // Adjoint windows of at most this many cells take the cooperative kernels: two steps and their
 // reverse take 744 ms there and 2,865 ms one cell per lane for 5,000 cells, 2,870 and 3,626 ms for
 // 20,000, 4,304 and 4,586 ms for 30,000.

@@ -6,7 +6,9 @@
 // that finishes its cell takes the next one at once, so a warp is no longer held by
 // its slowest cell.  The queue is ordered by each cell's step attempts in the previous
 // call, most first (a counting sort over step-count bins), so long cells start early
-// and the tail is short.  Every cell is integrated exactly as in k_chem_ros3; the
+// and the tail is short.  What is left when the queue has run dry is handed over to the
+// cooperative kernel (coop.cuh): a lane's attempt takes 1.3 ms however few lanes are busy, and
+// the cells with the most attempts took a third to a half of a call.  Every cell is integrated exactly as in k_chem_ros3; the
 // schedule changes no result bit.
 #pragma once
 #include <cuda_runtime.h>
@@ -17,12 +19,23 @@ namespace chem {
 
 constexpr int QUEUE_BINS = 256;
 
+// Cells that k_chem_ros3_queue leaves unfinished when its queue has run dry: their integrator
+// state, and the workspace (warp * 32 + lane) that holds Y (and its time integral).
+struct HandOver {
+    unsigned long long* count;        // zeroed before the launch
+    long long* cell;
+    int* slot;
+    ros3::CellState* state;
+    int most;                         // a block hands over what it has left once that is at most this (0: never)
+};
+
 struct QueueArgs {
     const int* order;                 // queue order of cells relative to cell0, or nullptr for 0, 1, ...
     unsigned long long* head;         // next queue position (zeroed before the launch)
     long long qlen;                   // cells in the queue (0: the whole grid)
     long long cell0;                  // first cell of the range the queue covers
     const unsigned long long* qlen_dev;   // if set: the queue length, written by an earlier kernel
+    HandOver over;                    // k_chem_ros3_queue: what it hands over; k_chem_ros3_coop: (count set) its queue
 };
 
 __device__ __forceinline__ unsigned long long queue_len(const QueueArgs& q, long long ncell)
@@ -78,7 +91,17 @@ __global__ void __launch_bounds__(WPB * 32, CHEM_QUEUE_WARPS_PER_SM / WPB > 0 ? 
         const bool busy = cell >= 0;
         bool night;
         if (LOCKSTEP) {
-            if (!__syncthreads_or(busy)) break;
+            const int left = __syncthreads_count(busy || !drained);
+            if (left == 0) break;
+            if (left <= q.over.most) {
+                if (busy) {
+                    const unsigned long long at = atomicAdd(q.over.count, 1ull);
+                    q.over.cell[at] = cell;
+                    q.over.slot[at] = (int)(warp * 32 + lane);
+                    q.over.state[at] = s;
+                }
+                break;
+            }
             night = __syncthreads_and(!busy || !sun) && a.use_night;
             CHEM_PHASE_MARK(s, 6);
         } else {

@@ -54,6 +54,9 @@ int cmaqchem_diag_fp64_issue(int device, int active_lanes, double* cycles_per_in
  * "ros3_coop" (ROS3: 1 the cooperative kernel, one cell per warp with its state in shared
  * memory, where the rate-constant pass's arrays were allocated, 0 one cell per lane, -1
  * (default) by the size of the call; same results) and
+ * "ros3_hand_over" (work-queue ROS3: a block whose queue has run dry leaves its last cells, once
+ * there are at most that many, to the cooperative kernel; 0 never, -1 (default) 3/8 of its lanes;
+ * where the rate-constant pass's arrays were allocated; same results) and
  * "adjoint_coop" (the adjoint's passes: 1 one cell per warp with its state in shared memory, 0 one
  * cell per lane, -1 (default) by the number of cells; the same states and gradients of a cell,
  * the rate gradients summed over the cells in another order) and

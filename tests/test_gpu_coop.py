@@ -114,6 +114,16 @@ def test_gear_cells_that_reach_the_evaluation_cap():
     same(run(s, t, -1, 1), a)
 
 
+@pytest.mark.parametrize("mech,dims", [("cb6r5_ae7_aq", (1, 1, 1)), ("cb6r5_ae7_aq", (37, 29, 3)), ("cracmm2", (31, 17, 2))])
+@pytest.mark.parametrize("most", [1, 64, 255])
+def test_cells_handed_over_by_the_work_queue(mech, dims, most):
+    _, t, s = setup(mech, dims, seed=34)
+    s.set_tuning(ros3_hand_over=0)
+    a = run(s, t, 0)
+    s.set_tuning(ros3_hand_over=most)
+    same(run(s, t, 0), a)
+
+
 def gradients(s, t, nsync, mode, tape_bytes=None):
     import torch
     from cmaq_gb300.adjoint import Ros3Window
