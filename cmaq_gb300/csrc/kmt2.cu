@@ -9,11 +9,13 @@
 // one Rodas3 attempt per pass of the kernel's loop (the phases of kmt2.cuh, with a block
 // barrier between them), and takes a new cell when its cell ends, so the lanes of a warp
 // stay busy while the cells' step counts differ.  A block leaves the loop when the queue is
-// empty and all its lanes are idle.  The integrator's loops are bounded (200,000 Rodas3
-// steps per pass, 5 step halvings per singular factorisation, 16 passes; a run of rejected
-// attempts shrinks h by 0.9 or more each until it is accepted or reaches 0, whose NaN error
-// norm is accepted as 1e-10), so every cell ends and so does every thread.
+// empty and few of its lanes are busy; the kernel of kmt2_coop.cuh goes on with their cells.
+// The integrator's loops are bounded (200,000 Rodas3 steps per pass, 5 step halvings per
+// singular factorisation, 16 passes; a run of rejected attempts shrinks h by 0.9 or more
+// each until it is accepted or reaches 0, whose NaN error norm is accepted as 1e-10), so
+// every cell ends and so does every thread.
 #include <cuda_runtime.h>
+#include <string.h>
 
 #include <algorithm>
 #include <string>
@@ -38,7 +40,7 @@ namespace {
 #endif
 constexpr int KMT2_THREADS = 128;
 constexpr long long KMT2_LANES_PER_SM = KMT2_THREADS * KMT2_MIN_BLOCKS;
-constexpr long long KMT2_WS_TAIL = 16;          // doubles after the lanes' slices: the queue counter
+constexpr long long KMT2_WS_TAIL = 16;          // doubles after the lanes' slices: the queue counters
 
 struct Kmt2Args {
     const double* params;
@@ -50,7 +52,20 @@ struct Kmt2Args {
     unsigned long long* next;   // the queue: cells handed out so far
     long long ncell;
     long long nlanes;           // a multiple of 32
+    int most;                   // the queue kernel: cells that a block leaves to the cooperative kernel at most
+    const double* left;         // the cooperative kernel: the lanes' slices with the cells left, or nullptr
 };
+
+// A cell left unfinished by the queue kernel: its number + 1 (0: none) and its variables, in the
+// place of the lane's GHIMJ, which the next attempt forms anew.
+struct Unfinished {
+    unsigned long long tag;
+    kmt2::Cell c;
+    kmt2::Lane L;
+    long long st[kmt2::NSTAT];
+};
+static_assert(sizeof(Unfinished) % 8 == 0 && sizeof(Unfinished) / 8 <= kmt2::LU_NONZERO, "room for a cell's variables");
+static_assert(sizeof(kmt2::Cell) == sizeof(kmt2w::Cell) && sizeof(kmt2::Lane) == sizeof(kmt2w::Lane), "one layout");
 
 // One pass of the warp's refill: the lanes with no cell (need) take consecutive cells of
 // the queue with one atomic per warp.  Returns the lane's new cell, or -1 when the queue is
@@ -73,7 +88,8 @@ __device__ __forceinline__ long long take_cell(bool need, unsigned long long* ne
 // with a block barrier between phases (KMT2_LOCKSTEP), so that the block's warps run the
 // same generated routine at the same time and share its instruction-cache lines; finish
 // (cell, c, L, st) writes a finished cell.  The block leaves the loop when, after a
-// refill, none of its lanes holds a cell (the queue is empty); a refill pass runs only
+// refill, the queue is empty and at most `most` of its lanes hold a cell, and leaves those
+// cells in their lanes' slices (Unfinished); a refill pass runs only
 // when KMT2_REFILL_MIN of the block's lanes are idle or none is busy.
 #ifndef KMT2_LOCKSTEP
 #define KMT2_LOCKSTEP 1
@@ -88,13 +104,13 @@ __device__ __forceinline__ long long take_cell(bool need, unsigned long long* ne
 #endif
 template <class Begin, class Finish>
 __device__ __forceinline__ void kmt2_queue_loop(bool has_ws, double* ws, unsigned long long* next, long long ncell,
-                                                Begin begin, Finish finish)
+                                                int most, Begin begin, Finish finish)
 {
     kmt2::Cell c;
     kmt2::Lane L;
     long long st[kmt2::NSTAT];
     long long cell = -1;
-    bool drained = !has_ws;
+    bool drained = !has_ws, empty = false;
     for (;;) {
         // refill when KMT2_REFILL_MIN lanes of the block are idle (or none is busy), so that
         // the set-up of new cells runs for several lanes at once
@@ -104,13 +120,15 @@ __device__ __forceinline__ void kmt2_queue_loop(bool has_ws, double* ws, unsigne
         const long long got = take_cell(need, next, ncell);
         if (need) {
             if (got < 0) {
-                drained = true;
+                drained = empty = true;
             } else {
                 cell = got;
                 begin(cell, c, L, st);
             }
         }
-        if (!__syncthreads_or(cell >= 0)) break;
+        const bool gone = __syncthreads_or(empty);   // the queue
+        const int left = __syncthreads_count(cell >= 0);
+        if (left == 0 || (gone && left <= most)) break;
         bool att = false;
         if (cell >= 0) {
             if (kmt2::kq_next(c, L, ws, st)) {
@@ -136,6 +154,42 @@ __device__ __forceinline__ void kmt2_queue_loop(bool has_ws, double* ws, unsigne
             kmt2::kq_decide(L, ws, st);
         }
     }
+    if (has_ws && most > 0) {
+        constexpr int WORDS = sizeof(Unfinished) / 8;
+        double* at = ws + kmt2::W_GHIMJ * kmt2::KQ_S;
+        if (cell < 0) {
+            *at = __longlong_as_double(0);
+        } else {
+            Unfinished u{};
+            u.tag = (unsigned long long)cell + 1;
+            u.c = c;
+            u.L = L;
+            for (int i = 0; i < kmt2::NSTAT; ++i) u.st[i] = st[i];
+            long long w[WORDS];
+            memcpy(w, &u, sizeof(u));
+            for (int i = 0; i < WORDS; ++i) at[i * kmt2::KQ_S] = __longlong_as_double(w[i]);
+        }
+    }
+}
+
+// The cell left in lane `pos` of the slices, for the warp that goes on with it: its workspace to ws, its
+// variables; -1: none.  The same in all lanes.
+__device__ __forceinline__ long long take_unfinished(const double* left, unsigned long long pos, double* ws,
+                                                     kmt2w::Cell& c, kmt2w::Lane& L, long long* st)
+{
+    constexpr int WORDS = sizeof(Unfinished) / 8;
+    const double* from = left + (pos >> 5) * (kmt2::KQ_S * kmt2::WS_ELEMS) + (pos & 31);
+    const double* at = from + kmt2::W_GHIMJ * kmt2::KQ_S;
+    if (__double_as_longlong(*at) == 0) return -1;
+    long long w[WORDS];
+    for (int i = 0; i < WORDS; ++i) w[i] = __double_as_longlong(at[i * kmt2::KQ_S]);
+    Unfinished u;
+    memcpy(&u, w, sizeof(u));
+    memcpy(&c, &u.c, sizeof(c));
+    memcpy(&L, &u.L, sizeof(L));
+    for (int i = 0; i < kmt2::NSTAT; ++i) st[i] = u.st[i];
+    for (int i = threadIdx.x & 31; i < kmt2::WS_ELEMS; i += 32) ws[i] = from[i * kmt2::KQ_S];
+    return (long long)u.tag - 1;
 }
 
 __global__ void __launch_bounds__(KMT2_THREADS, KMT2_MIN_BLOCKS) k_kmt2_queue(Kmt2Args a)
@@ -145,7 +199,7 @@ __global__ void __launch_bounds__(KMT2_THREADS, KMT2_MIN_BLOCKS) k_kmt2_queue(Km
     const long long n = a.ncell;
     constexpr long long s = kmt2::KQ_S;
     kmt2_queue_loop(
-        lane < a.nlanes, ws, a.next, n,
+        lane < a.nlanes, ws, a.next, n, a.most,
         [&](long long cell, kmt2::Cell& c, kmt2::Lane& L, long long* st) {
             kmt2::kq_begin(c, L, a.params + cell, n, a.var_mix + cell, n, a.params[kmt2::P_HO * n + cell], ws, st);
         },
@@ -175,6 +229,8 @@ struct AqchemArgs {
     int naer;
     int ai[kmt2::KA_NIDX];
     double fac[kmt2::KF_N];
+    int most;               // as in Kmt2Args
+    const double* left;
 };
 
 // the whole AQCHEM: a new cell is mapped into the KPP state (kq_aq_map) before its set-up, a
@@ -185,7 +241,7 @@ __global__ void __launch_bounds__(KMT2_THREADS, KMT2_MIN_BLOCKS) k_aqchem_queue(
     double* ws = a.ws + (lane >> 5) * (kmt2::KQ_S * kmt2::WS_ELEMS) + (lane & 31);
     const long long n = a.ncell;
     kmt2_queue_loop(
-        lane < a.nlanes, ws, a.next, n,
+        lane < a.nlanes, ws, a.next, n, a.most,
         [&](long long cell, kmt2::Cell& c, kmt2::Lane& L, long long* st) {
             kmt2::kq_aq_map(a.params + cell, a.gas + cell, a.aer + cell, a.naer, a.ai, a.fac, n, ws);
             kmt2::kq_begin(c, L, a.params + cell, n, ws + kmt2::W_YNEW * kmt2::KQ_S, kmt2::KQ_S,
@@ -204,7 +260,11 @@ __global__ void __launch_bounds__(kmt2_coop::Coop::MAX_CELLS * 32, 1) k_kmt2_coo
     using namespace kmt2w;
     const long long n = a.ncell;
     kmt2_coop::integrate(
-        smem, a.next, n,
+        smem, a.next, a.left ? a.nlanes : n,
+        [&](unsigned long long pos, Cell& c, Lane& L, long long* st, double* ws) {
+            return take_unfinished(a.left, pos, ws, c, L, st);
+        },
+        a.left != nullptr,
         [&](long long cell, Cell& c, double* ws) {
             return kq_setup(c, a.params + cell, n, a.var_mix + cell, n, a.params[P_HO * n + cell], ws + W_Y, ws + W_F,
                             ws + W_R);
@@ -225,7 +285,11 @@ __global__ void __launch_bounds__(kmt2_coop::Coop::MAX_CELLS * 32, 1) k_aqchem_c
     using namespace kmt2w;
     const long long n = a.ncell;
     kmt2_coop::integrate(
-        smem, a.next, n,
+        smem, a.next, a.left ? a.nlanes : n,
+        [&](unsigned long long pos, Cell& c, Lane& L, long long* st, double* ws) {
+            return take_unfinished(a.left, pos, ws, c, L, st);
+        },
+        a.left != nullptr,
         [&](long long cell, Cell& c, double* ws) {
             kq_aq_map(a.params + cell, a.gas + cell, a.aer + cell, a.naer, a.ai, a.fac, n, ws);
             return kq_setup(c, a.params + cell, n, ws + W_YNEW, KQ_S, a.gas[KG_HO * n + cell], ws + W_Y, ws + W_F,
@@ -244,25 +308,42 @@ int fail(const std::string& msg)
     return -1;
 }
 
-// Whether a call takes the cooperative kernels (same results): 333 cells take 12.8 ms there and
-// 148 one cell per lane, 4,000 cells 40 and 165 ms, 25,000 cells 225 and 277 ms; at 100,000 cells
-// the lanes are full: 880 and 661 ms.
-constexpr long long COOP_LIMIT = 35000;
+// Whether a call takes the cooperative kernels from the start (same results): 333 cells take 12.8 ms
+// there and 148 one cell per lane, 5,000 cells 54 and 105 ms (by the queue kernel with what it
+// leaves), 15,000 cells 149 and 155, 25,000 cells 243 and 203, 100,000 cells 952 and 540 ms.
+constexpr long long COOP_LIMIT = 16000;
 bool use_coop(long long ncell) { return ncell <= COOP_LIMIT; }
 
+// A call's kernels: cooperative, or the queue kernel and then the cooperative one for the cells that its
+// blocks leave once the queue is empty and at most KMT2_LEAVE of their 128 lanes are busy: a lane's
+// step takes 3 ms however few there are.  25,000 and 100,000 cells take 281 and 687 ms when none is
+// left, 230 / 596 with 16, 220 / 556 with 32, 205 / 527 with 64, 203 / 540 with 80, 200 / 559 with 100.
+constexpr int KMT2_LEAVE = 80;
+
 template <class Args>
-cudaError_t launch_coop(void (*kernel)(Args), const Args& a, cudaStream_t s)
+cudaError_t launch(void (*queue)(Args), void (*cooperative)(Args), Args a, long long blocks, cudaStream_t s)
 {
     int dev = 0, nsm = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaMemsetAsync(a.next, 0, 2 * sizeof(unsigned long long), s);
     if (e != cudaSuccess) return e;
-    const int cells = (int)std::min<long long>(kmt2_coop::Coop::MAX_CELLS, (a.ncell + nsm - 1) / nsm);
-    const int nb = (int)std::min<long long>(nsm, (a.ncell + cells - 1) / cells);
+    long long n = a.ncell;
+    if (!use_coop(n)) {
+        a.most = KMT2_LEAVE;
+        queue<<<(unsigned)blocks, KMT2_THREADS, 0, s>>>(a);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        a.left = a.ws;
+        a.next = a.next + 1;
+        n = blocks * a.most;
+    }
+    const int cells = (int)std::min<long long>(kmt2_coop::Coop::MAX_CELLS, (n + nsm - 1) / nsm);
+    const int nb = (int)std::min<long long>(nsm, (n + cells - 1) / cells);
     const size_t bytes = coop::smem_bytes<kmt2_coop::Coop>(cells);
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    e = cudaFuncSetAttribute(cooperative, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;
-    kernel<<<nb, cells * 32, bytes, s>>>(a);
+    cooperative<<<nb, cells * 32, bytes, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -311,15 +392,8 @@ extern "C" int cmaqchem_kmt2_solve_device(long long ncell, const double* params,
     const long long blocks = kmt2_lanes(ncell, workspace, workspace_doubles, &nlanes, &next);
     if (blocks < 0) return -1;
     cudaStream_t s = (cudaStream_t)stream;
-    cudaError_t e = cudaMemsetAsync(next, 0, sizeof(unsigned long long), s);
-    if (e != cudaSuccess) return fail(std::string("queue counter: ") + cudaGetErrorString(e));
-    Kmt2Args a{params, var_mix, var_out, fix_out, stats, workspace, next, ncell, nlanes};
-    if (use_coop(ncell)) {
-        e = launch_coop(k_kmt2_coop, a, s);
-    } else {
-        k_kmt2_queue<<<(unsigned)blocks, KMT2_THREADS, 0, s>>>(a);
-        e = cudaGetLastError();
-    }
+    const Kmt2Args a{params, var_mix, var_out, fix_out, stats, workspace, next, ncell, nlanes, 0, nullptr};
+    cudaError_t e = launch(k_kmt2_queue, k_kmt2_coop, a, blocks, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(std::string("k_kmt2_queue: ") + cudaGetErrorString(e));
     return 0;
@@ -389,8 +463,6 @@ extern "C" int cmaqchem_aqchem_device(long long ncell, const double* params, dou
     const long long blocks = kmt2_lanes(ncell, workspace, workspace_doubles, &nlanes, &next);
     if (blocks < 0) return -1;
     cudaStream_t s = (cudaStream_t)stream;
-    cudaError_t e = cudaMemsetAsync(next, 0, sizeof(unsigned long long), s);
-    if (e != cudaSuccess) return fail(std::string("queue counter: ") + cudaGetErrorString(e));
     a.params = params;
     a.gas = gas;
     a.aer = aerosol;
@@ -403,12 +475,7 @@ extern "C" int cmaqchem_aqchem_device(long long ncell, const double* params, dou
     a.ncell = ncell;
     a.nlanes = nlanes;
     a.naer = naer;
-    if (use_coop(ncell)) {
-        e = launch_coop(k_aqchem_coop, a, s);
-    } else {
-        k_aqchem_queue<<<(unsigned)blocks, KMT2_THREADS, 0, s>>>(a);
-        e = cudaGetLastError();
-    }
+    cudaError_t e = launch(k_aqchem_queue, k_aqchem_coop, a, blocks, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(std::string("k_aqchem_queue: ") + cudaGetErrorString(e));
     return 0;

@@ -226,12 +226,13 @@ __device__ __forceinline__ void decide(double* ws, Lane& L, long long* st)
         if (i < NVAR) { __VA_ARGS__ }                        \
     }
 
-// The cells of a call: the block's warps take cells from the queue and go through the steps
+// The cells of a call: the block's warps take cells from the queue of `count` and go through the steps
 // together.  begin(cell, ws): lane 0's set-up of a new cell, its status; finish(cell, c, L, st, ws): its
-// write-back, by the whole warp.
-template <class Begin, class Finish>
-__device__ __forceinline__ void integrate(char* smem, unsigned long long* next, long long ncell, Begin begin,
-                                          Finish finish)
+// write-back, by the whole warp.  resuming: the queue's positions are lanes that may have left a
+// cell, which resume(pos, c, L, st, ws) brings here (-1: none).
+template <class Resume, class Begin, class Finish>
+__device__ __forceinline__ void integrate(char* smem, unsigned long long* next, long long count, Resume resume,
+                                          bool resuming, Begin begin, Finish finish)
 {
     const int lane = threadIdx.x & 31;
     double* cst = (double*)(smem + Coop::TABLE_SMEM);
@@ -251,19 +252,24 @@ __device__ __forceinline__ void integrate(char* smem, unsigned long long* next, 
     for (;;) {
         if (cell < 0 && !drained) {   // the same in all lanes
             unsigned long long pos = 0;
-            if (lane == 0) pos = atomicAdd(next, 1ull);
-            pos = __shfl_sync(0xffffffffu, pos, 0);
-            if (pos < (unsigned long long)ncell) {
-                cell = (long long)pos;
+            do {
+                if (lane == 0) pos = atomicAdd(next, 1ull);
+                pos = __shfl_sync(0xffffffffu, pos, 0);
+                if (resuming && pos < (unsigned long long)count) cell = resume(pos, c, L, st, ws);
+            } while (resuming && cell < 0 && pos < (unsigned long long)count);
+            if (pos < (unsigned long long)count) {
                 int e = 0;
-                if (lane == 0) e = begin(cell, shared_cell, ws);
-                e = __shfl_sync(0xffffffffu, e, 0);
-                __syncwarp();
-                c = shared_cell;
-                for (int i = 0; i < NSTAT; ++i) st[i] = 0;
-                L.tc = 0.0;
-                L.ierr = e != 0 ? e - 100 : 1;
-                L.phase = e != 0 ? KL_DONE : KL_PASS;
+                if (!resuming) {
+                    cell = (long long)pos;
+                    if (lane == 0) e = begin(cell, shared_cell, ws);
+                    e = __shfl_sync(0xffffffffu, e, 0);
+                    __syncwarp();
+                    c = shared_cell;
+                    for (int i = 0; i < NSTAT; ++i) st[i] = 0;
+                    L.tc = 0.0;
+                    L.ierr = e != 0 ? e - 100 : 1;
+                    L.phase = e != 0 ? KL_DONE : KL_PASS;
+                }
                 if (e == 0) {
                     factors(ws, c);
                     e3[0] = kq_exp(0.0 * c.delinvt);

@@ -45,3 +45,19 @@ def test_aqchem_same_bits_as_one_cell_per_lane(n, ispc8):
         out.append([x.cpu().numpy()[:, :n] for x in (gas, aer, *rest)])
     for x, y in zip(*out):
         assert np.array_equal(x, y, equal_nan=True)
+
+
+@pytest.mark.parametrize("copies", [40000, 90001])
+def test_cells_that_the_queue_kernel_leaves(copies):
+    """The last cells of a call that does not take the cooperative kernels go on there: every copy ends alike."""
+    from cmaq_gb300.aqchem import aqchem
+    n = 1217
+    p, g, a, index, fac = make_cloud_columns(n, seed=43, mtpyrac=1)
+    p[11, 1] = 0.0                          # a failed set-up
+    out = []
+    for idx in (np.arange(n), np.arange(copies) % n):
+        gas, aer = up(g[idx].T), up(a[idx].T)
+        rest = aqchem(up(p[idx].T), gas, aer, index, fac)
+        out.append([x.cpu().numpy() for x in (gas, aer, *rest)])
+    for x, y in zip(*out):
+        assert np.array_equal(x[:, np.arange(copies) % n], y, equal_nan=True)
