@@ -631,11 +631,12 @@ __device__ __forceinline__ void corrector_rhs(double* __restrict__ ws, double de
 }
 
 // The f evaluation a cell asked for, with its predictor matrix first and its corrector
-// solve after (day pattern, see the file comment).
-template <class M, int S>
+// solve after (day pattern, see the file comment), of one cell per lane; a warp's lanes go
+// through the programs of gear_coop.cuh instead.
+template <class M, int S, bool COOP>
 __device__ __forceinline__ void evaluate(double* __restrict__ ws, const State& s, bool go)
 {
-    constexpr bool COOP = false;
+    static_assert(!COOP, "one cell per lane");
     if (go && s.need_jac) {
         M::gear_explic_0(ws);
         M::gear_pdecomp_0(ws, s.r1delt);
@@ -749,7 +750,7 @@ __global__ void __launch_bounds__(GEAR_WPB * 32, GEAR_WARPS_PER_SM / GEAR_WPB) k
             cell = -1;
             busy = false;
         }
-        gear::evaluate<M, 32>(ws, s, busy);
+        gear::evaluate<M, 32, false>(ws, s, busy);
     }
     if (a.counters) {
         for (int o = 16; o > 0; o >>= 1) {
