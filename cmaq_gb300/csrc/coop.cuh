@@ -524,6 +524,8 @@ __global__ void __launch_bounds__(C::MAX_CELLS * 32, 1) k_chem_ros3_coop(chem::G
     }
 }
 
+// A launch asks for its cells' bytes; the kernel's limit is always set to MAX_CELLS' (a limit per
+// launch would be another thread's, which launches on a handle of its own).
 template <class C>
 inline size_t smem_bytes(int cells)
 {

@@ -341,7 +341,8 @@ cudaError_t launch(void (*queue)(Args), void (*cooperative)(Args), Args a, long 
     const int cells = (int)std::min<long long>(kmt2_coop::Coop::MAX_CELLS, (n + nsm - 1) / nsm);
     const int nb = (int)std::min<long long>(nsm, (n + cells - 1) / cells);
     const size_t bytes = coop::smem_bytes<kmt2_coop::Coop>(cells);
-    e = cudaFuncSetAttribute(cooperative, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    e = cudaFuncSetAttribute(cooperative, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)coop::smem_bytes<kmt2_coop::Coop>(kmt2_coop::Coop::MAX_CELLS));
     if (e != cudaSuccess) return e;
     cooperative<<<nb, cells * 32, bytes, s>>>(a);
     return cudaGetLastError();

@@ -131,7 +131,8 @@ struct MechOps {
     {                                                                                               \
         const size_t bytes = coop::smem_bytes<NS::CoopEbi>(cells);                                  \
         cudaError_t r = cudaFuncSetAttribute(chem::k_chem_ebi_warp<T_, NS::CoopEbi>,                \
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); \
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize,           \
+                                             (int)coop::smem_bytes<NS::CoopEbi>(NS::CoopEbi::MAX_CELLS)); \
         if (r != cudaSuccess) return r;                                                             \
         chem::k_chem_ebi_warp<T_, NS::CoopEbi><<<nb, cells * 32, bytes, s>>>(a, q, e);              \
         return cudaGetLastError();                                                                  \
@@ -167,7 +168,8 @@ struct MechOps {
         const size_t bytes = coop::smem_bytes<R>(cells);                                            \
         const void* f = reverse ? (const void*)coop::k_adj_reverse_coop<T_, R>                      \
                                 : (const void*)coop::k_adj_forward_coop<T_, F>;                     \
-        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); \
+        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,        \
+                                             (int)coop::smem_bytes<R>(R::MAX_CELLS));               \
         if (e != cudaSuccess) return e;                                                             \
         if (reverse) coop::k_adj_reverse_coop<T_, R><<<nb, cells * 32, bytes, s>>>(a);              \
         else coop::k_adj_forward_coop<T_, F><<<nb, cells * 32, bytes, s>>>(a);                      \
@@ -247,7 +249,8 @@ struct MechOps {
     {                                                                                               \
         const size_t bytes = coop::smem_bytes<NS::Coop>(cells);                                     \
         cudaError_t r = cudaFuncSetAttribute(coop::k_chem_ros3_coop<T_, NS::Coop>,                  \
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); \
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize,           \
+                                             (int)coop::smem_bytes<NS::Coop>(NS::Coop::MAX_CELLS)); \
         if (r != cudaSuccess) return r;                                                             \
         coop::k_chem_ros3_coop<T_, NS::Coop><<<nb, cells * 32, bytes, s>>>(a, q);                   \
         return cudaGetLastError();                                                                  \
