@@ -254,7 +254,8 @@ int cmaqchem_ros3_solve_noalloc(const char* mechanism, long long ncell, double* 
  * handle; the caller supplies a device workspace of cmaqchem_kmt2_workspace_doubles(nlanes)
  * doubles (nlanes >= 1): nlanes threads integrate the cells, each taking the next cell
  * of a queue (a counter at the end of the workspace, cleared on `stream` by the call)
- * when its cell ends, so one call's workspace serves any ncell.  Device arrays,
+ * when its cell ends, so one call's workspace serves any ncell.  Calls of at most 16,000
+ * cells, and the last cells of larger ones, run one cell per warp in shared memory instead.  Device arrays,
  * [element][cell]:
  *   params  [CMAQCHEM_KMT2_NPARAM][ncell]: TEMP2 (K), PRES_PA (Pa), TAUCLD (s), PRCRATE (mm/h),
  *           WCAVG, WTAVG (kg/m3), AIRM (mol/m2), ALFA0, ALFA3 (1/s), COSZEN, JH2O2 (1/s),
