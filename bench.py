@@ -1029,7 +1029,8 @@ def main():
         except Exception:
             traffic = None
     if rank == 0:
-        launches_per_step = 4   # queue ordering (hist, scan, scatter) + solve, replayed from one graph
+        # queue ordering (hist, scan, scatter), rates, solve (and ROS3's last cells), replayed from one graph
+        launches_per_step = 6 if a.solver == "ros3" else 5
         if a.solver != "ros3":   # EBI iterations and Gear steps have no ROS3 FLOP count
             achieved_tf = None
         bclk = (batched["clocks"] or {}).get("sm_mhz")

@@ -604,8 +604,9 @@ static int enqueue_step(cmaqchem_handle* h, const chem::GridArgs& a, int itmstep
                 CK(h->ops->ebi_rconst_pass(a, c0, c1, h->d_rki_all, h->d_sun_all, h->nblocks, s));
                 // A call lasts at least as long as its slowest cell, whose iterations take longer
                 // the more warps share the SM: one per sub-partition up to 256 cells per SM (27,880
-                // CB6r5 cells: 288 ms with 4 warps, 347 with 8, 383 with 10), above that 8 (200,000
-                // cells: 1,064, 668 and 626 ms; a later call of the hour 212, 149 and 165 ms).
+                // CB6r5 cells: 259 ms with 4 warps, 268 with 6, 272 with 8), above that 8 (200,000
+                // cells with 4, 8 and 10: 1,064, 668 and 626 ms; a later call of the hour 212, 149 and
+                // 165 ms).
                 const long long share = (n + h->nsm - 1) / h->nsm;
                 const int cells = (int)std::min<long long>(share <= 256 ? 4 : std::min(8, h->ops->ebi_max_cells), share);
                 const int nb = (int)std::min<long long>(h->nsm, (n + cells - 1) / cells);

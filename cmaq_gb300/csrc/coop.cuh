@@ -308,7 +308,8 @@ __device__ __forceinline__ void run(S& st, int rows, uint32_t cell, uint32_t cst
 
 // One attempt of ros3::attempt_phased (rbsolver.F:344-589) on the warp's cell; the scalar state
 // is kept identically by the lanes.  Every warp of the block calls it; one with
-// active == false goes through the rows on whatever its cell holds.  yave: the cell's
+// active == false leaves the FP64 pipe to the others (27,880 EBI cells 270 -> 259 ms, 12 ROS3 calls of
+// 10,527 cells 148 -> 146 ms).  yave: the cell's
 // time integral of Y in global memory (stride ystride), or nullptr.  ADJ: of the adjoint's forward pass.
 template <class M, class C, bool ADJ = false>
 __device__ __forceinline__ void attempt(double* __restrict__ x, Stream<C>& rows, uint32_t cst, ros3::CellState& s,
@@ -333,7 +334,7 @@ __device__ __forceinline__ void attempt(double* __restrict__ x, Stream<C>& rows,
     const double dtinv = fpdiv::div(1.0, dt);
     if (sub == 0) x[C::G] = dtinv * RGAM;
     // f(Y), the factors, stage 1: V = -K1
-    run<C>(rows, C::STAGE1_ROWS, cell, cst);
+    run<C>(rows, C::STAGE1_ROWS, cell, cst, active);
     // The species loops run the same trips in every lane: lanes that left a loop early went
     // through the rows that follow apart from the others, at twice the time.
 #pragma unroll
@@ -345,7 +346,7 @@ __device__ __forceinline__ void attempt(double* __restrict__ x, Stream<C>& rows,
             x[C::T + n] = x[C::Y + n] + k1;
         }
     }
-    run<C>(rows, C::RHS_ROWS, cell, cst);
+    run<C>(rows, C::RHS_ROWS, cell, cst, active);
     {
         const double x1 = C21 * dtinv;
 #pragma unroll
@@ -354,7 +355,7 @@ __device__ __forceinline__ void attempt(double* __restrict__ x, Stream<C>& rows,
             if (n < N) x[C::V + n] = fma(-x1, x[C::K1 + n], -x[C::T + n]);
         }
     }
-    run<C>(rows, C::SOLVE_ROWS, cell, cst);
+    run<C>(rows, C::SOLVE_ROWS, cell, cst, active);
     {   // stage 3
         const double x1 = C31 * dtinv;
         const double x2 = C32 * dtinv;
@@ -369,7 +370,7 @@ __device__ __forceinline__ void attempt(double* __restrict__ x, Stream<C>& rows,
             }
         }
     }
-    run<C>(rows, C::SOLVE_ROWS, cell, cst);
+    run<C>(rows, C::SOLVE_ROWS, cell, cst, active);
     // solution (T) and weighted error (K1) of each species, then the norm in species order
     int bad = 0;
 #pragma unroll 1

@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(E::MAX_CELLS * 32, 1) k_chem_ebi_warp(GridArgs
             if (lane == 0) x[E::DTC] = s.dtc;
         }
         __syncwarp();
-        coop::run<E>(rows, E::ITERATION_ROWS, cell0, cst0);
+        coop::run<E>(rows, E::ITERATION_ROWS, cell0, cst0, go);
         if (!rows.ok) {   // a table chunk did not arrive: the cell fails
             s.status |= ebi::ST_MAXITER;
             s.done = true;
