@@ -112,7 +112,7 @@ struct cmaqchem_handle {
     int ebi_warp = 1;        // EBI: 1 one cell per warp (shared memory), 0 one cell per lane
     int ebi_defer = 0;       // EBI: > 0 one cell per lane, cells past this many iterations per warp
                              // (100, the best of 20-800, takes 491 and 885 ms where the warps alone
-                             // take 288 and 668 ms for 27,880 and 200,000 CB6r5 cells)
+                             // take 270 and 668 ms for 27,880 and 200,000 CB6r5 cells)
     int* d_ebi_def = nullptr;
     unsigned long long* d_ebi_ndef = nullptr;
     size_t ws_warps = 0;     // workspace capacity in warps

@@ -11,7 +11,7 @@
 // coop.cuh), the rest divisions and the species loops.  The earlier warp kernel walked index
 // tables in global memory and ran the group solutions HRG1-HRG4 on one lane: 0.2 ms.  A first
 // call of 27,880 CB6r5 cells took 881 ms with it and the one-cell-per-lane kernel for the
-// quick cells, and takes 288 ms here.
+// quick cells, and takes 259-272 ms here.
 #pragma once
 #include "coop.cuh"
 #include "ebi.cuh"
