@@ -77,6 +77,7 @@ def lib(variant: str = "default") -> C.CDLL:
     L.cmaqchem_diag_fp64_peak_long.argtypes = [C.c_int, C.c_double, C.POINTER(C.c_double), C.POINTER(C.c_double)]
     L.cmaqchem_diag_set_tuning.argtypes = [vp, C.c_char_p, C.c_int]
     L.cmaqchem_diag_fp64_rate.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_double)]
+    L.cmaqchem_diag_starved_rows.argtypes = [C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int)]
     L.cmaqchem_diag_phase_cycles.argtypes = [C.c_int, C.POINTER(C.c_ulonglong), C.c_int]
     L.cmaqchem_kmt2_workspace_doubles.argtypes = [C.c_longlong]
     L.cmaqchem_kmt2_workspace_doubles.restype = C.c_longlong
@@ -142,3 +143,12 @@ def mech_info(mechanism: str):
     order = (C.c_int * info.nspec)()
     check(lib().cmaqchem_mech_info_get(mechanism.encode(), None, order))
     return info, list(order)
+
+
+def starved_rows(feed: bool, chunks: int, device: int = 0) -> list[bool]:
+    """Per thread of a block whose table rows stop coming after `chunks` chunks: whether its waits went well."""
+    out = (C.c_int * 96)()
+    n = lib().cmaqchem_diag_starved_rows(device, int(feed), int(chunks), out)
+    if n < 0:
+        raise ChemError("starved rows probe failed")
+    return [bool(v) for v in out[:n]]

@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(C::MAX_CELLS * 32, 1) k_adj_reverse_coop(adj::
     }
     rows.drain();
     for (int r = sub; r < M::NRXNS; r += 32) {
-        const double v = x[C::GK + r];
+        const double v = rows.ok ? x[C::GK + r] : NAN;
         if (v != 0.0) atomicAdd(&a.grad_logk[r], v);
     }
     if (a.counters && ncells && sub == 0) atomicAdd(&a.counters[1], ncells);

@@ -56,39 +56,76 @@ __device__ __forceinline__ uint2 ldw(uint32_t p)
     return v;
 }
 
-// Waits, with a limit, for the phase of an mbarrier to complete.
-__device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t parity)
+__device__ __forceinline__ bool try_parity(uint32_t bar, uint32_t parity)
 {
-    uint32_t done = 0;
-    for (int tries = 0; !done && tries < 1 << 20; ++tries)
-        asm volatile("{ .reg .pred q; mbarrier.try_wait.parity.shared.b64 q, [%1], %2; selp.u32 %0, 1, 0, q; }"
-                     : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    uint32_t done;
+    asm volatile("{ .reg .pred q; mbarrier.try_wait.parity.shared.b64 q, [%1], %2; selp.u32 %0, 1, 0, q; }"
+                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     return done != 0;
 }
+// The chunk of turn t was not there at once: whether it arrives within some `limit` cycles, the same in
+// all lanes of the warp.  When it does not, what is in flight to the two buffers has had that time again
+// when this returns, and the mark behind the block's barriers spares its warps later waits.
+static __device__ __noinline__ bool wait_longer(uint32_t bar, uint32_t t, long long limit)
+{
+    uint32_t mark;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(mark) : "r"(bar + 16) : "memory");
+    if (__any_sync(0xffffffffu, mark != 0)) return false;
+    const auto wait = [&](bool both) {
+        bool there = false;
+        for (const long long t0 = clock64(); !there && __all_sync(0xffffffffu, clock64() - t0 < limit);) {
+            there = try_parity(bar + 8 * (t & 1u), t >> 1 & 1u);
+            if (both) there = try_parity(bar + 8 * ((t + 1) & 1u), (t + 1) >> 1 & 1u) && there;
+            there = __all_sync(0xffffffffu, there);
+        }
+        return there;
+    };
+    if (wait(false)) return true;
+    wait(true);
+    asm volatile("st.shared.u32 [%0], %1;" : : "r"(bar + 16), "r"(1u) : "memory");
+    return false;
+}
+
+// How a chunk of a table travels: one bulk copy, whose arrival completes the barrier's phase.
+struct BulkCopy {
+    static constexpr long long LIMIT = 1ll << 31;   // a wait gives up after a second
+    __device__ __forceinline__ void operator()(uint32_t to, const uint2* from, uint32_t bytes, uint32_t bar)
+    {
+        asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" : : "r"(bar), "r"(bytes) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     : : "r"(to), "l"(from), "r"(bytes), "r"(bar) : "memory");
+    }
+};
 
 // The block's stream of table rows: chunks of CHUNK rows, fetched by one bulk copy each into
 // two buffers in shared memory that all warps read, in the order of one pass through the
 // programs (C::chunk), and again.  A warp that fetched its rows itself waited for the L2 on
 // every row.
-template <class C>
+//
+// A chunk that does not arrive ends the stream: `ok` turns false in all lanes of a warp at once
+// (no lane waits in a vote of the warp for one that gave up), and the kernels report every cell that the
+// warp takes from then on as failed.  Thread 0 fetches only while its own warp has seen every chunk,
+// so no buffer is fetched into while a copy to it is under way; when it stops, the other warps' next
+// waits end too.  All warps keep to the block's barriers throughout.  What a chunk that is there does
+// not need lies out of line (with `ok` tested before the wait, a vote of the block at the release, or
+// the wait inline, some calls took up to 5 % more time).
+template <class C, class Copy = BulkCopy>
 struct Stream {
     static constexpr int W = 32;
     static constexpr uint32_t BYTES = C::CHUNK * W * 8;
     static constexpr uint32_t PITCH = (C::CHUNK + AHEAD) * W * 8;   // rows of zeros end a buffer: looked ahead at only
-    uint32_t buf, bar;   // shared addresses: two buffers, two barriers
+    uint32_t buf, bar;   // shared addresses: two buffers; two barriers and the mark of wait_longer
     int k;               // chunk of the pass
     uint32_t turn;       // chunks taken so far
     bool ok;             // false: a copy did not arrive (the wait gave up)
+    Copy copy;
 
     __device__ __forceinline__ static int wrap(int c) { return c >= C::PASS ? c - C::PASS : c; }
 
     // thread 0: the copy of the pass's chunk c into buffer i
     __device__ __forceinline__ void fetch(int c, uint32_t i)
     {
-        const uint2* src = C::rows() + (size_t)C::chunk(c) * (C::CHUNK * W);
-        asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" : : "r"(bar + 8 * i), "r"(BYTES) : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                     : : "r"(buf + PITCH * i), "l"(src), "r"(BYTES), "r"(bar + 8 * i) : "memory");
+        copy(buf + PITCH * i, C::rows() + (size_t)C::chunk(c) * (C::CHUNK * W), BYTES, bar + 8 * i);
     }
 
     // smem: C::TABLE_SMEM bytes, 128-byte aligned.  Called by the whole block.
@@ -102,6 +139,7 @@ struct Stream {
         for (uint32_t j = threadIdx.x; j < 2 * AHEAD * W; j += blockDim.x)
             *(uint2*)((char*)smem + PITCH * (j / (AHEAD * W)) + BYTES + 8 * (j % (AHEAD * W))) = make_uint2(0u, 0u);
         if (threadIdx.x == 0) {
+            asm volatile("st.shared.u32 [%0], %1;" : : "r"(bar + 16), "r"(0u) : "memory");
             asm volatile("mbarrier.init.shared.b64 [%0], 1;" : : "r"(bar) : "memory");
             asm volatile("mbarrier.init.shared.b64 [%0], 1;" : : "r"(bar + 8) : "memory");
             asm volatile("fence.mbarrier_init.release.cluster;" : : : "memory");
@@ -112,19 +150,25 @@ struct Stream {
         __syncthreads();
     }
 
+    // whether the chunk of turn t has arrived, the same in all lanes of the warp
+    __device__ __forceinline__ bool arrived(uint32_t t)
+    {
+        if (__all_sync(0xffffffffu, try_parity(bar + 8 * (t & 1u), t >> 1 & 1u))) return true;
+        return wait_longer(bar, t, Copy::LIMIT);
+    }
+
     // waits (with a limit) for the current chunk and returns its shared address
     __device__ __forceinline__ uint32_t wait()
     {
-        const uint32_t i = turn & 1u;
-        if (!wait_parity(bar + 8 * i, turn >> 1 & 1u)) ok = false;
-        return buf + PITCH * i;
+        if (!arrived(turn)) ok = false;
+        return buf + PITCH * (turn & 1u);
     }
 
     // the block is through with the current chunk: its buffer takes the one after the next
     __device__ __forceinline__ void release()
     {
         __syncthreads();
-        if (threadIdx.x == 0) {
+        if (threadIdx.x == 0 && ok) {
             asm volatile("fence.proxy.async.shared::cta;" : : : "memory");
             fetch(wrap(k + 2), turn & 1u);
         }
@@ -135,29 +179,27 @@ struct Stream {
     // the copies in flight have arrived (a block must not end before them)
     __device__ __forceinline__ void drain()
     {
-        wait();
-        ++turn;
-        wait();
+        if (!ok) return;
+        arrived(turn);
+        arrived(turn + 1);
     }
 };
 
 // The rows of a one-warp block that goes through its programs by demand: begin names the
-// chunks to come, cancel drops those not taken.
-template <class C>
+// chunks to come, cancel drops those not taken.  It ends as a Stream does.
+template <class C, class Copy = BulkCopy>
 struct Feed {
     static constexpr int W = 32;
     static constexpr uint32_t BYTES = C::CHUNK * W * 8, PITCH = (C::CHUNK + AHEAD) * W * 8;
     uint32_t buf, bar, turn;
     int next, end;       // chunk to take next, end of what was begun
     bool ok;
+    Copy copy;
 
     __device__ __forceinline__ void fetch(int c, uint32_t i)
     {
-        const uint2* src = C::rows() + (size_t)c * (C::CHUNK * W);
         asm volatile("fence.proxy.async.shared::cta;" : : : "memory");
-        asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" : : "r"(bar + 8 * i), "r"(BYTES) : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                     : : "r"(buf + PITCH * i), "l"(src), "r"(BYTES), "r"(bar + 8 * i) : "memory");
+        copy(buf + PITCH * i, C::rows() + (size_t)c * (C::CHUNK * W), BYTES, bar + 8 * i);
     }
 
     __device__ __forceinline__ void init(void* smem)
@@ -170,6 +212,7 @@ struct Feed {
         for (uint32_t j = threadIdx.x; j < 2 * AHEAD * W; j += W)
             *(uint2*)((char*)smem + PITCH * (j / (AHEAD * W)) + BYTES + 8 * (j % (AHEAD * W))) = make_uint2(0u, 0u);
         if (threadIdx.x == 0) {
+            asm volatile("st.shared.u32 [%0], %1;" : : "r"(bar + 16), "r"(0u) : "memory");
             asm volatile("mbarrier.init.shared.b64 [%0], 1;" : : "r"(bar) : "memory");
             asm volatile("mbarrier.init.shared.b64 [%0], 1;" : : "r"(bar + 8) : "memory");
             asm volatile("fence.mbarrier_init.release.cluster;" : : : "memory");
@@ -180,6 +223,7 @@ struct Feed {
     // chunks [c0, c1): the first two are on their way when it returns
     __device__ __forceinline__ void begin(int c0, int c1)
     {
+        if (!ok) return;
         next = c0;
         end = c1;
         __syncwarp();
@@ -189,16 +233,22 @@ struct Feed {
         }
     }
 
+    __device__ __forceinline__ bool arrived(uint32_t t)
+    {
+        if (__all_sync(0xffffffffu, try_parity(bar + 8 * (t & 1u), t >> 1 & 1u))) return true;
+        return wait_longer(bar, t, Copy::LIMIT);
+    }
+
     __device__ __forceinline__ uint32_t wait()
     {
-        const uint32_t i = turn & 1u;
-        if (!wait_parity(bar + 8 * i, turn >> 1 & 1u)) ok = false;
-        return buf + PITCH * i;
+        if (!arrived(turn)) ok = false;
+        return buf + PITCH * (turn & 1u);
     }
 
     __device__ __forceinline__ void release()
     {
         __syncwarp();
+        if (!ok) return;
         if (threadIdx.x == 0 && next + 2 < end) fetch(next + 2, turn & 1u);
         ++turn;
         ++next;
@@ -207,7 +257,7 @@ struct Feed {
     __device__ __forceinline__ void cancel()
     {
         for (int n = min(2, end - next); n > 0; --n) {
-            wait();
+            if (!arrived(turn)) ok = false;
             ++turn;
         }
         next = end = 0;

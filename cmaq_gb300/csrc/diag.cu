@@ -4,6 +4,8 @@
 #include <string>
 
 #include "../../include/cmaqchem_diag.h"
+#include "coop.cuh"
+#include "gen/cb6r5_ae7_aq_coop.cuh"
 
 #ifdef CHEM_PHASE_TIMING
 // clock cycles per phase of the lock-stepped ROS3 attempt (ros3.cuh: CHEM_PHASE_MARK)
@@ -214,4 +216,72 @@ extern "C" int cmaqchem_diag_fp64_rate(int device, int op, int chains, int threa
     *ops_per_clk_per_sm = ops / (t * 1.0e-3) / nsm / (khz * 1.0e3);
     if (ms) *ms = t;
     return 0;
+}
+
+namespace {
+
+using Rows = mech_cb6r5_ae7_aq::Coop;
+constexpr int STARVED_WARPS = 3, STARVED_CHUNKS = 4;
+
+// Copies for the first `left` chunks only; the barriers of later ones stay armed, and a wait gives up
+// after a millisecond.
+struct Starved {
+    static constexpr long long LIMIT = 1ll << 21;
+    int left;
+    __device__ __forceinline__ void operator()(uint32_t to, const uint2* from, uint32_t bytes, uint32_t bar)
+    {
+        if (left-- > 0) coop::BulkCopy()(to, from, bytes, bar);
+        else asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" : : "r"(bar), "r"(bytes) : "memory");
+    }
+};
+
+// STARVED_CHUNKS chunks of rows on cells of zeros from a stream (or a one-warp block's feed) of which
+// `chunks` arrive: out[thread] = whether its waits went well
+template <bool FEED>
+__global__ void k_starved(int chunks, int* out)
+{
+    extern __shared__ __align__(128) char starved_smem[];
+    double* cst = (double*)(starved_smem + Rows::TABLE_SMEM);
+    double* x = cst + Rows::NCONST + (size_t)(threadIdx.x / 32) * Rows::ELEMS;
+    for (int i = threadIdx.x; i < Rows::NCONST; i += blockDim.x) cst[i] = Rows::constants()[i];
+    for (int i = threadIdx.x & 31; i < Rows::ELEMS; i += 32) x[i] = 0.0;
+    const uint32_t cell = (uint32_t)__cvta_generic_to_shared(x), c0 = (uint32_t)__cvta_generic_to_shared(cst);
+    bool ok;
+    if constexpr (FEED) {
+        coop::Feed<Rows, Starved> rows;
+        rows.copy.left = chunks;
+        rows.init(starved_smem);
+        rows.begin(0, STARVED_CHUNKS + 1);
+        coop::run<Rows>(rows, STARVED_CHUNKS * Rows::CHUNK, cell, c0);
+        ok = rows.ok;
+        rows.cancel();
+    } else {
+        coop::Stream<Rows, Starved> rows;
+        rows.copy.left = chunks;
+        rows.start(starved_smem);
+        coop::run<Rows>(rows, STARVED_CHUNKS * Rows::CHUNK, cell, c0);
+        ok = rows.ok;
+        rows.drain();
+    }
+    out[threadIdx.x] = ok;
+}
+
+}  // namespace
+
+extern "C" int cmaqchem_diag_starved_rows(int device, int feed, int chunks, int* out)
+{
+    if (chunks < 0 || !out || cudaSetDevice(device) != cudaSuccess) return -1;
+    const int threads = feed ? 32 : 32 * STARVED_WARPS;
+    const int bytes = (int)coop::smem_bytes<Rows>(feed ? 1 : STARVED_WARPS);
+    const void* f = feed ? (const void*)k_starved<true> : (const void*)k_starved<false>;
+    int* d = nullptr;
+    cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) e = cudaMalloc(&d, sizeof(int) * threads);
+    if (e != cudaSuccess) return -1;
+    if (feed) k_starved<true><<<1, threads, bytes>>>(chunks, d);
+    else k_starved<false><<<1, threads, bytes>>>(chunks, d);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpy(out, d, sizeof(int) * threads, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? threads : -1;
 }

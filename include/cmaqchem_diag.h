@@ -36,6 +36,12 @@ int cmaqchem_diag_fp64_rate(int device, int op, int chains, int threads, int blo
  * (1-32) lanes active: the latency a cell's sequential FP64 work pays per operation. */
 int cmaqchem_diag_fp64_issue(int device, int active_lanes, double* cycles_per_instruction);
 
+/* The table stream of the cooperative kernels (feed 0: a block of three warps) or the feed of the
+ * one-warp SMVGEAR blocks (feed 1) when only the first `chunks` of the four chunks of rows that it
+ * takes arrive: out[thread] whether the thread's waits went well.  Returns the number of threads (at
+ * most 96), or -1. */
+int cmaqchem_diag_starved_rows(int device, int feed, int chunks, int* out);
+
 /* Scheduling knobs of a handle, for the autotuner: "night_pattern" (1: warps whose cells are
  * all dark use the smaller night LU pattern; 0: the day pattern always, same numbers),
  * "lockstep" (work-queue kernel: 0 free-running warps, 1 (default) the block's warps run
