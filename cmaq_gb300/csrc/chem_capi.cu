@@ -110,9 +110,8 @@ struct cmaqchem_handle {
     int q_nblocks = 0;
     int q_bps_cap = 0;       // blocks per SM of the queue kernel, 0: as many as fit
     int ebi_warp = 1;        // EBI: 1 one cell per warp (shared memory), 0 one cell per lane
-    int ebi_defer = 0;       // EBI: > 0 one cell per lane, cells past this many iterations per warp
-                             // (100, the best of 20-800, takes 491 and 885 ms where the warps alone
-                             // take 270 and 668 ms for 27,880 and 200,000 CB6r5 cells)
+    int ebi_defer = -1;      // EBI: > 0 one cell per lane, cells past this many iterations per warp; -1:
+                             // ebi_defer_of
     int* d_ebi_def = nullptr;
     unsigned long long* d_ebi_ndef = nullptr;
     size_t ws_warps = 0;     // workspace capacity in warps
@@ -235,6 +234,18 @@ int configure_queue(cmaqchem_handle* h)
         }
     }
     return 0;
+}
+
+// Iterations after which an EBI cell goes from its lane to a warp (0: the warps take all cells).  With
+// the rates of a pass the warps alone are the fastest: 270 and 668 ms for a first call of 27,880 and
+// 200,000 CB6r5 cells, against 491 and 885 ms with 100 iterations, the best of 20-800.  Where
+// there was no room for the pass (a large grid) a warp has its rates from one lane: 27,880 and 126,000
+// CB6r5 cells take 338 and 766 ms with the warps alone, 353 and 640 ms with 100, and 3,961 and
+// 4,999 ms one cell per lane to the end; 11,200 and 72,000 CRACMM2 cells 374 and 1,005, 422 and
+// 1,051, 4,099 and 8,959 ms.
+int ebi_defer_of(const cmaqchem_handle* h, bool pass)
+{
+    return h->ebi_defer >= 0 ? h->ebi_defer : h->ebi_warp && !pass ? 100 : 0;
 }
 
 // Whether a ROS3 call of n cells takes the cooperative kernel (same results): below the
@@ -397,6 +408,7 @@ extern "C" int cmaqchem_init(const cmaqchem_cfg* cfg, cmaqchem_handle** out)
             if (upload_gear_coef(h)) return -1;
         }
         if (cfg->solver == CMAQCHEM_SOLVER_EBI) {
+            if (ensure_ws(h, (size_t)h->nsm * m->ebi_max_cells)) return -1;   // for rates without the pass
             CK(cudaMalloc(&h->d_ebi_def, sizeof(int) * h->ncell));
             CK(cudaMalloc(&h->d_ebi_ndef, sizeof(unsigned long long)));
         }
@@ -511,8 +523,8 @@ extern "C" int cmaqchem_diag_set_tuning(cmaqchem_handle* h, const char* key, int
         h->graph_exec = nullptr;
         return 0;
     } else if (strcmp(key, "rconst_pass") == 0) {
-        // 1: the work-queue ROS3 call evaluates CALC_RCONST in a pass of whole warps first
-        // (when its arrays were allocated at set-up); 0: in the refilled lanes; same numbers
+        // 1: a call evaluates CALC_RCONST in a pass of whole warps first (when its arrays were
+        // allocated at set-up); 0: the solver kernel does, cell by cell; same numbers
         h->rconst_pass = value != 0;
         if (h->graph_exec) CK(cudaGraphExecDestroy(h->graph_exec));
         h->graph_exec = nullptr;
@@ -577,12 +589,13 @@ static int enqueue_step(cmaqchem_handle* h, const chem::GridArgs& a, int itmstep
             q.order = h->d_order + c0;
         }
         CK(cudaMemsetAsync(h->d_head, 0, sizeof(unsigned long long), s));
+        const bool pass = h->rconst_pass && h->d_rki_all;
         if (gear_solver) {
             chem::GearArgs g{};
             g.coef = h->d_gear_coef;
             if (h->gear_warp) {
                 chem::GridArgs ap = a;
-                if (h->d_rki_all) {
+                if (pass) {
                     CK(h->ops->rconst_pass(a, c0, c1, h->d_rki_all, h->d_sun_all, h->nblocks, s));
                     ap.rki_all = h->d_rki_all;
                     ap.sun_all = h->d_sun_all;
@@ -599,9 +612,11 @@ static int enqueue_step(cmaqchem_handle* h, const chem::GridArgs& a, int itmstep
             // the cells of [c0, c1), or those of a deferred list: one cell per warp, few to a block
             auto by_warps = [&](const chem::QueueArgs& qw, const chem::EbiArgs& ew) -> int {
                 chem::GridArgs ap = a;
-                ap.rki_all = h->d_rki_all;
-                ap.sun_all = h->d_sun_all;
-                CK(h->ops->ebi_rconst_pass(a, c0, c1, h->d_rki_all, h->d_sun_all, h->nblocks, s));
+                if (pass) {
+                    ap.rki_all = h->d_rki_all;
+                    ap.sun_all = h->d_sun_all;
+                    CK(h->ops->ebi_rconst_pass(a, c0, c1, h->d_rki_all, h->d_sun_all, h->nblocks, s));
+                }
                 // A call lasts at least as long as its slowest cell, whose iterations take longer
                 // the more warps share the SM: one per sub-partition up to 256 cells per SM (27,880
                 // CB6r5 cells: 259 ms with 4 warps, 268 with 6, 272 with 8), above that 8 (200,000
@@ -613,12 +628,11 @@ static int enqueue_step(cmaqchem_handle* h, const chem::GridArgs& a, int itmstep
                 CK(h->ops->chem_ebi_warp(ap, qw, ew, cells, nb, s));
                 return 0;
             };
-            if (!h->d_rki_all) {   // no room for the rates of the call: one cell per lane
-                CK(h->ops->chem_ebi(a, q, e, h->nblocks, s));
-            } else if (h->ebi_defer > 0) {
-                // one cell per lane for the cells that finish within ebi_defer iterations,
+            const int defer = ebi_defer_of(h, pass);
+            if (defer > 0) {
+                // one cell per lane for the cells that finish within `defer` iterations,
                 // then one cell per warp for the others
-                e.defer_after = h->ebi_defer;
+                e.defer_after = defer;
                 e.deferred = h->d_ebi_def;
                 e.ndeferred = h->d_ebi_ndef;
                 CK(cudaMemsetAsync(h->d_ebi_ndef, 0, sizeof(unsigned long long), s));
@@ -633,7 +647,7 @@ static int enqueue_step(cmaqchem_handle* h, const chem::GridArgs& a, int itmstep
             } else {
                 CK(h->ops->chem_ebi(a, q, e, h->nblocks, s));
             }
-        } else if (h->rconst_pass && h->d_rki_all) {
+        } else if (pass) {
             CK(h->ops->rconst_pass(a, c0, c1, h->d_rki_all, h->d_sun_all, h->nblocks, s));
             chem::GridArgs ap = a;
             ap.rki_all = h->d_rki_all;

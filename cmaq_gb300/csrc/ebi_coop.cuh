@@ -36,6 +36,22 @@ __global__ void __launch_bounds__(THREADS_PER_BLOCK, 1) k_ebi_rconst_pass(GridAr
     }
 }
 
+// The rate constants of the warp's cell without that pass, by its first lane; returns the sunlight
+// flag.  Out of line: the iterations' code stays as it is.
+template <class M>
+__device__ __noinline__ bool ebi_rates_of_cell(const GridArgs& a, long long cell, double* __restrict__ rki)
+{
+    const int lane = threadIdx.x & 31;
+    const size_t warp = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    double* ws = a.ws + warp * ((size_t)M::WS_ELEMS * 32);   // the first lane's column
+    int sun = 0;
+    if (lane == 0) sun = rconst_cell_ebi<M>(a, cell, ws) ? 1 : 0;
+    sun = __shfl_sync(0xffffffffu, sun, 0);
+    __syncwarp();
+    for (int r = lane; r < M::NRXNS; r += 32) rki[r] = ws[(M::OFF_RKI + r) * 32];
+    return sun != 0;
+}
+
 // What follows an iteration's program in ebi::iterate: the species updates, the convergence
 // test and HRSOLVER's bookkeeping.  notmax: the lane's species' NOTMAX flags (bit i: species
 // lane + 32 i).
@@ -129,8 +145,9 @@ __device__ __forceinline__ void ebi_coop_update(double* __restrict__ x, ebi::Sta
     __syncwarp();
 }
 
-// One EBI CHEM call, a cell per warp from the work queue (rates from k_ebi_rconst_pass).  The
-// block's warps go through the iterations together.  Dynamic shared memory as k_chem_ros3_coop's.
+// One EBI CHEM call, a cell per warp from the work queue.  Rates come from k_ebi_rconst_pass or,
+// without its arrays, from the warp's first lane in its column of the workspace, while the block
+// waits.  The block's warps go through the iterations together.  Dynamic shared memory as k_chem_ros3_coop's.
 template <class M, class E>
 __global__ void __launch_bounds__(E::MAX_CELLS * 32, 1) k_chem_ebi_warp(GridArgs a, QueueArgs q, EbiArgs e)
 {
@@ -166,8 +183,12 @@ __global__ void __launch_bounds__(E::MAX_CELLS * 32, 1) k_chem_ebi_warp(GridArgs
                     x[E::YC0 + i] = x[E::YCP + i] = x[E::PROD + i] = x[E::LOSS + i] = x[E::PNEG + i] = 0.0;
                     if (v <= ebi::MAXPRED) notmax |= 1u << (i >> 5);
                 }
-                for (int r = lane; r < M::NRXNS; r += 32) x[E::RKI + r] = a.rki_all[(size_t)r * a.ncell + cell];
-                sun = a.sun_all[cell] != 0;
+                if (a.rki_all) {
+                    for (int r = lane; r < M::NRXNS; r += 32) x[E::RKI + r] = a.rki_all[(size_t)r * a.ncell + cell];
+                    sun = a.sun_all[cell] != 0;
+                } else {
+                    sun = ebi_rates_of_cell<M>(a, cell, x + E::RKI);
+                }
                 s.tmstep = e.tmstep;
                 s.dtc = e.tmstep;
                 s.n_ebi_steps = e.n_ebi_steps;

@@ -88,7 +88,12 @@ typedef struct {
 } cmaqchem_mech_info;
 
 /* Replaces the first-call set-up of CHEM: RBINIT, RBSPARSE, RESET_SPECIES_POINTERS
- * (rbdriver.F:226-371).  Allocates device tables and workspaces for the domain. */
+ * (rbdriver.F:226-371).  Allocates device tables and workspaces for the domain.  Beside the
+ * workspaces (a few GB, whatever the domain) the largest are the rate constants of a call, nrxns
+ * doubles per cell (2,792 bytes with cb6r5_ae7_aq, 4,256 with cracmm2: 13.4 and 20.4 GB for 4.8
+ * million cells), held by every handle but a ROS3 one of the static schedule for more cells than its
+ * cooperative kernels take; when they would not leave a quarter of the free device memory, the
+ * solvers evaluate the rates cell by cell instead, with the same results. */
 int cmaqchem_init(const cmaqchem_cfg* cfg, cmaqchem_handle** out);
 
 /* One CHEM call on host arrays (rbdriver.F:373-785): copies the inputs to the device,

@@ -53,10 +53,9 @@ int cmaqchem_diag_starved_rows(int device, int feed, int chunks, int* out);
  * consecutive cells; 0 (default): the largest step's tape, halved until it fits) and
  * "ros3_dtmin_exp" (ROS3's minimum step is 10^value minutes; default -8, the reference's
  * DTMIN; a lower value lets tight tolerances pass the initial radical transient) and
- * "rconst_pass" (1, default when its arrays fit at set-up: the work-queue ROS3 call
- * evaluates CALC_RCONST of every cell in a pass of whole warps before the solver kernel,
- * which gathers the rates; 0: the solver kernel evaluates them in the lanes it refills;
- * same results) and
+ * "rconst_pass" (1, default when its arrays fit at set-up: a call evaluates CALC_RCONST of
+ * every cell in a pass of whole warps before the solver kernel, which gathers the rates;
+ * 0: the solver kernel evaluates them cell by cell; same results) and
  * "ros3_coop" (ROS3: 1 the cooperative kernel, one cell per warp with its state in shared
  * memory, where the rate-constant pass's arrays were allocated, 0 one cell per lane, -1
  * (default) by the size of the call; same results) and
@@ -73,8 +72,8 @@ int cmaqchem_diag_starved_rows(int device, int feed, int chunks, int* out);
  * "ebi_warp" (EBI solver: 1 (default) one cell per warp with its state in shared memory,
  * 0 one cell per lane; same results), "ebi_defer" (EBI: n > 0 runs one cell per lane and
  * hands the cells still iterating after n Backward-Euler iterations to the one-cell-per-warp
- * kernel, which integrates them from their inputs; 0 (default): ebi_warp alone decides;
- * same results) and
+ * kernel, which integrates them from their inputs; 0: ebi_warp alone decides; by default 0
+ * with the rate-constant pass and 100 without it; same results) and
  * "gear_warp" (SMVGEAR: 1 (default) one cell per warp with its workspace in shared memory,
  * 0 one cell per lane; same results). */
 struct cmaqchem_handle;
