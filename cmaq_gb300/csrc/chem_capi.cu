@@ -1043,13 +1043,14 @@ int adj_setup(cmaqchem_handle* h, long long ncell)
     return 0;
 }
 
-// The forward or reverse sweep of a queue of cells: cooperative up to the mechanism's limit,
+// The forward or reverse sweep of a queue of cells: cooperative up to the mechanism's limit for it,
 // above it one cell per lane (the same states, tapes and gradients of a cell), whose
 // workspaces are allocated by the first call that needs them.
 cudaError_t adj_launch(cmaqchem_handle* h, const adj::Args& a, bool reverse, cudaStream_t s)
 {
     const long long n = a.queue_len > 0 ? a.queue_len : a.ncell;
-    if (h->adj_coop >= 0 ? h->adj_coop > 0 : n <= h->ops->adj_coop_limit) return h->ops->adj_coop(a, reverse, h->nsm, s);
+    const long long limit = reverse ? h->ops->adj_reverse_coop_limit : h->ops->adj_coop_limit;
+    if (h->adj_coop >= 0 ? h->adj_coop > 0 : n <= limit) return h->ops->adj_coop(a, reverse, h->nsm, s);
     if (!h->d_adj_ws) {
         int fb = 0, rb = 0;
         cudaError_t e = h->ops->adj_occupancy(&fb, &rb);

@@ -63,8 +63,8 @@ struct MechOps {
     int coop_max_cells;
     long long coop_limit;
     cudaError_t (*chem_coop)(const chem::GridArgs&, const chem::QueueArgs&, int cells, int nblocks, cudaStream_t);
-    // cooperative adjoint kernels, taken for at most adj_coop_limit cells
-    long long adj_coop_limit;
+    // cooperative adjoint kernels, taken for at most this many cells by the forward and the reverse sweep
+    long long adj_coop_limit, adj_reverse_coop_limit;
     cudaError_t (*adj_coop)(const adj::Args&, bool reverse, int nsm, cudaStream_t);
 };
 
@@ -276,4 +276,4 @@ struct MechOps {
                                    T_::ADJ_WS_ELEMS, adj_forward_, adj_reverse_, adj_occupancy_, ddm_update_,     \
                                    rconst_, rconst_pass_, occupancy_, T_::GEAR_WS_ELEMS, gear_, gear_occupancy_, \
                                    gear_warp_, gear_warp_occupancy_, NS::Coop::MAX_CELLS, NS::COOP_LIMIT, chem_coop_, \
-                                   NS::ADJ_COOP_LIMIT, adj_coop_};
+                                   NS::ADJ_COOP_LIMIT, NS::ADJ_REVERSE_COOP_LIMIT, adj_coop_};
