@@ -1035,32 +1035,38 @@ int grow(T** p, size_t* cap, size_t need)
     return 0;
 }
 
+// Whether a sweep over n cells takes the cooperative kernels: up to the mechanism's limit for it
+bool adj_use_coop(const cmaqchem_handle* h, long long n, bool reverse)
+{
+    return h->adj_coop >= 0 ? h->adj_coop > 0
+                            : n <= (reverse ? h->ops->adj_reverse_coop_limit : h->ops->adj_coop_limit);
+}
+
+// What a call over ncell cells needs, before it sizes a tape by the free memory: the workspaces of the
+// one-cell-per-lane kernels (1.8 GB) too, when one of its sweeps over all cells takes them (sweeps
+// over batches of fewer cells take them only when that one does).
 int adj_setup(cmaqchem_handle* h, long long ncell)
 {
     if (!h->d_adj_counters) CK(cudaMalloc(&h->d_adj_counters, 3 * sizeof(unsigned long long)));
     if (grow(&h->d_adj_order, &h->adj_cell_cap, (size_t)ncell)) return -1;
     if (grow(&h->d_adj_status, &h->adj_status_cap, (size_t)ncell)) return -1;
-    return 0;
-}
-
-// The forward or reverse sweep of a queue of cells: cooperative up to the mechanism's limit for it,
-// above it one cell per lane (the same states, tapes and gradients of a cell), whose
-// workspaces are allocated by the first call that needs them.
-cudaError_t adj_launch(cmaqchem_handle* h, const adj::Args& a, bool reverse, cudaStream_t s)
-{
-    const long long n = a.queue_len > 0 ? a.queue_len : a.ncell;
-    const long long limit = reverse ? h->ops->adj_reverse_coop_limit : h->ops->adj_coop_limit;
-    if (h->adj_coop >= 0 ? h->adj_coop > 0 : n <= limit) return h->ops->adj_coop(a, reverse, h->nsm, s);
-    if (!h->d_adj_ws) {
+    if (!h->d_adj_ws && !(adj_use_coop(h, ncell, false) && adj_use_coop(h, ncell, true))) {
         int fb = 0, rb = 0;
-        cudaError_t e = h->ops->adj_occupancy(&fb, &rb);
-        if (e != cudaSuccess) return e;
+        CK(h->ops->adj_occupancy(&fb, &rb));
         int bps = fb < rb ? fb : rb;
         if (bps < 1) bps = 1;
         h->adj_nblocks = h->nsm * bps;
-        e = cudaMalloc(&h->d_adj_ws, (size_t)h->adj_nblocks * adj::WPB * h->ops->adj_ws_elems * 32 * sizeof(double));
-        if (e != cudaSuccess) return e;
+        CK(cudaMalloc(&h->d_adj_ws, (size_t)h->adj_nblocks * adj::WPB * h->ops->adj_ws_elems * 32 * sizeof(double)));
     }
+    return 0;
+}
+
+// The forward or reverse sweep of a queue of cells, cooperative or one cell per lane (the same
+// states, tapes and gradients of a cell).
+cudaError_t adj_launch(cmaqchem_handle* h, const adj::Args& a, bool reverse, cudaStream_t s)
+{
+    const long long n = a.queue_len > 0 ? a.queue_len : a.ncell;
+    if (adj_use_coop(h, n, reverse)) return h->ops->adj_coop(a, reverse, h->nsm, s);
     adj::Args b = a;
     b.ws = h->d_adj_ws;
     return reverse ? h->ops->adj_reverse(b, h->adj_nblocks, s) : h->ops->adj_forward(b, h->adj_nblocks, s);

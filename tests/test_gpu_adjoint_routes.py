@@ -38,3 +38,36 @@ def test_one_route_forward_the_other_back(mech, cells, tape_bytes):
             assert np.array_equal(a, b)
         # sums over the cells, in another order: the largest gradient stands for the sum of magnitudes
         assert np.max(np.abs(got[3] - lanes[3])) <= 1e-10 * np.max(np.abs(lanes[3]))
+
+
+def test_backward_when_the_tape_fills_the_memory():
+    """A backward call that takes the one-cell-per-lane kernels on a handle that has not taken them before, with so
+    much memory free that its tape fits alone but not beside their workspaces (1.8 GB): the tape gives way."""
+    import torch
+    from cmaq_gb300.adjoint import Ros3Window
+    from cmaq_gb300.chem import ChemSolver
+    mech, cells = "cb6r5_ae7_aq", 70000
+    window(mech, 33, 0, 0, 0)                  # the kernels' own memory
+    g = make_grid(mech, cells, 1, 1, seed=84)
+    got = []
+    for room in (None, 900 << 20):
+        with ChemSolver(mech, ncols=cells, nrows=1, nlays=1, nspcsd=g.nspcsd, cgrid_index=g.cgrid_index, rtol=1e-3,
+                        atol=1e-9) as s:
+            y0, rki, night = solver_inputs(g, s)
+            w = Ros3Window(s, rki, night, 1, 5.0, tape_bytes=0)
+            x = y0.clone().requires_grad_(True)
+            s.set_tuning(adjoint_coop=1)
+            y = w(x)
+            s.set_tuning(adjoint_coop=0)
+            held = None
+            if room is not None:
+                tape = int(y.grad_fn.saved_tensors[1].sum()) * (s.info.ischan + 1) * 8
+                assert tape > 1800 << 20       # so that half of it and the workspaces fit
+                torch.cuda.empty_cache()
+                held = torch.empty(torch.cuda.mem_get_info()[0] - tape - room, dtype=torch.uint8, device="cuda")
+            try:
+                got.append(torch.autograd.grad(y.sum(), x)[0].cpu().numpy())
+            finally:
+                del held
+                torch.cuda.empty_cache()       # for the tests that follow
+    assert np.array_equal(got[0], got[1])
