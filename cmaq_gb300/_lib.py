@@ -77,6 +77,7 @@ def lib(variant: str = "default") -> C.CDLL:
     L.cmaqchem_diag_fp64_peak_long.argtypes = [C.c_int, C.c_double, C.POINTER(C.c_double), C.POINTER(C.c_double)]
     L.cmaqchem_diag_set_tuning.argtypes = [vp, C.c_char_p, C.c_int]
     L.cmaqchem_diag_fp64_rate.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_double)]
+    L.cmaqchem_diag_step_factor.argtypes = [C.c_int, C.c_longlong, vp, vp, vp]
     L.cmaqchem_diag_starved_rows.argtypes = [C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int)]
     L.cmaqchem_diag_phase_cycles.argtypes = [C.c_int, C.POINTER(C.c_ulonglong), C.c_int]
     L.cmaqchem_kmt2_workspace_doubles.argtypes = [C.c_longlong]
@@ -143,6 +144,17 @@ def mech_info(mechanism: str):
     order = (C.c_int * info.nspec)()
     check(lib().cmaqchem_mech_info_get(mechanism.encode(), None, order))
     return info, list(order)
+
+
+def step_factor(maxerr, device: int = 0):
+    """ROS3's step factor of an accepted step on the device, float64 array in: (as the forward kernels
+    form it, by pow)."""
+    import numpy as np
+    x = np.ascontiguousarray(maxerr, dtype=np.float64)
+    out = np.empty((2, x.size))
+    if lib().cmaqchem_diag_step_factor(device, x.size, x.ctypes.data, out[0].ctypes.data, out[1].ctypes.data) != 0:
+        raise ChemError("step factor probe failed")
+    return out[0], out[1]
 
 
 def starved_rows(feed: bool, chunks: int, device: int = 0) -> list[bool]:

@@ -268,6 +268,35 @@ __global__ void k_starved(int chunks, int* out)
 
 }  // namespace
 
+namespace {
+
+__global__ void k_step_factor(long long n, const double* maxerr, double* refined, double* by_pow)
+{
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        refined[i] = ros3::step_factor<false>(maxerr[i]);
+        by_pow[i] = ros3::step_factor<true>(maxerr[i]);
+    }
+}
+
+}  // namespace
+
+extern "C" int cmaqchem_diag_step_factor(int device, long long n, const double* maxerr, double* refined, double* by_pow)
+{
+    if (n < 1 || !maxerr || !refined || !by_pow || cudaSetDevice(device) != cudaSuccess) return -1;
+    double* d = nullptr;
+    const size_t bytes = sizeof(double) * (size_t)n;
+    if (cudaMalloc(&d, 3 * bytes) != cudaSuccess) return -1;
+    cudaError_t e = cudaMemcpy(d, maxerr, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        k_step_factor<<<256, 256>>>(n, d, d + n, d + 2 * n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(refined, d + n, bytes, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(by_pow, d + 2 * n, bytes, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? 0 : -1;
+}
+
 extern "C" int cmaqchem_diag_starved_rows(int device, int feed, int chunks, int* out)
 {
     if (chunks < 0 || !out || cudaSetDevice(device) != cudaSuccess) return -1;

@@ -36,6 +36,10 @@ int cmaqchem_diag_fp64_rate(int device, int op, int chains, int threads, int blo
  * (1-32) lanes active: the latency a cell's sequential FP64 work pays per operation. */
 int cmaqchem_diag_fp64_issue(int device, int active_lanes, double* cycles_per_instruction);
 
+/* The step factor 0.9 / maxerr^(1/3) of an accepted ROS3 step for n values (host arrays): as the
+ * forward kernels form it, and by pow as the adjoint's do. */
+int cmaqchem_diag_step_factor(int device, long long n, const double* maxerr, double* refined, double* by_pow);
+
 /* The table stream of the cooperative kernels (feed 0: a block of three warps) or the feed of the
  * one-warp SMVGEAR blocks (feed 1) when only the first `chunks` of the four chunks of rows that it
  * takes arrive: out[thread] whether the thread's waits went well.  Returns the number of threads (at
