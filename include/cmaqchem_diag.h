@@ -61,8 +61,9 @@ int cmaqchem_diag_starved_rows(int device, int feed, int chunks, int* out);
  * every cell in a pass of whole warps before the solver kernel, which gathers the rates;
  * 0: the solver kernel evaluates them cell by cell; same results) and
  * "ros3_coop" (ROS3: 1 the cooperative kernel, one cell per warp with its state in shared
- * memory, where the rate-constant pass's arrays were allocated, 0 one cell per lane, -1
- * (default) by the size of the call; same results) and
+ * memory, where the rate-constant pass's arrays were allocated, 0 the kernel of the schedule, one
+ * cell per lane up to what "ros3_hand_over" leaves of it, -1 (default) by the size of the call;
+ * same results) and
  * "ros3_hand_over" (work-queue ROS3: a block whose queue has run dry leaves its last cells, once
  * there are at most that many, to the cooperative kernel; 0 never, -1 (default) 3/8 of its lanes;
  * where the rate-constant pass's arrays were allocated; same results) and
