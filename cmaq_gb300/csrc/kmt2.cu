@@ -21,6 +21,7 @@
 #include <string>
 
 #include "../../include/cmaqchem.h"
+#include "../../include/cmaqchem_diag.h"
 #include "kmt2.cuh"
 #include "kmt2_coop.cuh"
 
@@ -320,8 +321,9 @@ bool use_coop(long long ncell) { return ncell <= COOP_LIMIT; }
 // left, 230 / 596 with 16, 220 / 556 with 32, 205 / 527 with 64, 203 / 540 with 80, 200 / 559 with 100.
 constexpr int KMT2_LEAVE = 80;
 
+// route: CMAQCHEM_KMT2_BY_SIZE, or one kernel for every cell (cmaqchem_diag.h)
 template <class Args>
-cudaError_t launch(void (*queue)(Args), void (*cooperative)(Args), Args a, long long blocks, cudaStream_t s)
+cudaError_t launch(void (*queue)(Args), void (*cooperative)(Args), Args a, long long blocks, int route, cudaStream_t s)
 {
     int dev = 0, nsm = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -329,11 +331,11 @@ cudaError_t launch(void (*queue)(Args), void (*cooperative)(Args), Args a, long 
     if (e == cudaSuccess) e = cudaMemsetAsync(a.next, 0, 2 * sizeof(unsigned long long), s);
     if (e != cudaSuccess) return e;
     long long n = a.ncell;
-    if (!use_coop(n)) {
-        a.most = KMT2_LEAVE;
+    if (route == CMAQCHEM_KMT2_BY_SIZE ? !use_coop(n) : route != CMAQCHEM_KMT2_COOP) {
+        a.most = route == CMAQCHEM_KMT2_LANES ? 0 : KMT2_LEAVE;
         queue<<<(unsigned)blocks, KMT2_THREADS, 0, s>>>(a);
         e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+        if (e != cudaSuccess || a.most == 0) return e;
         a.left = a.ws;
         a.next = a.next + 1;
         n = blocks * a.most;
@@ -381,10 +383,11 @@ extern "C" long long cmaqchem_kmt2_workspace_doubles(long long nlanes)
     return nlanes > 0 ? (nlanes + 31) / 32 * 32 * (long long)kmt2::WS_ELEMS + KMT2_WS_TAIL : 0;
 }
 
-extern "C" int cmaqchem_kmt2_solve_device(long long ncell, const double* params, const double* var_mix,
-                                          double* var_out, double* fix_out, int* stats, double* workspace,
-                                          long long workspace_doubles, void* stream)
+extern "C" int cmaqchem_diag_kmt2_solve(int route, long long ncell, const double* params, const double* var_mix,
+                                        double* var_out, double* fix_out, int* stats, double* workspace,
+                                        long long workspace_doubles, void* stream)
 {
+    if (route < CMAQCHEM_KMT2_BY_SIZE || route > CMAQCHEM_KMT2_HAND_OVER) return fail("unknown route");
     if (ncell < 0) return fail("ncell must be >= 0");
     if (ncell == 0) return 0;
     if (!params || !var_mix || !var_out || !stats || !workspace) return fail("null array argument");
@@ -394,10 +397,18 @@ extern "C" int cmaqchem_kmt2_solve_device(long long ncell, const double* params,
     if (blocks < 0) return -1;
     cudaStream_t s = (cudaStream_t)stream;
     const Kmt2Args a{params, var_mix, var_out, fix_out, stats, workspace, next, ncell, nlanes, 0, nullptr};
-    cudaError_t e = launch(k_kmt2_queue, k_kmt2_coop, a, blocks, s);
+    cudaError_t e = launch(k_kmt2_queue, k_kmt2_coop, a, blocks, route, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(std::string("k_kmt2_queue: ") + cudaGetErrorString(e));
     return 0;
+}
+
+extern "C" int cmaqchem_kmt2_solve_device(long long ncell, const double* params, const double* var_mix,
+                                          double* var_out, double* fix_out, int* stats, double* workspace,
+                                          long long workspace_doubles, void* stream)
+{
+    return cmaqchem_diag_kmt2_solve(CMAQCHEM_KMT2_BY_SIZE, ncell, params, var_mix, var_out, fix_out, stats, workspace,
+                                    workspace_doubles, stream);
 }
 
 // Host-array form for callers without device arrays (a Fortran cloud module): the same
@@ -442,11 +453,12 @@ extern "C" int cmaqchem_kmt2_solve(long long ncell, const double* params, const 
 
 // The whole AQCHEM for a batch of cloudy cells: GAS / AEROSOL in, the KPP state, the kinetic
 // core, GAS / AEROSOL / wet deposition out (include/cmaqchem.h: cmaqchem_aqchem_device).
-extern "C" int cmaqchem_aqchem_device(long long ncell, const double* params, double* gas, double* aerosol, int naer,
-                                      const int* aer_index, const double* factors, double* gas_wdep,
-                                      double* aer_wdep, double* out, int* stats, double* workspace,
-                                      long long workspace_doubles, void* stream)
+extern "C" int cmaqchem_diag_aqchem(int route, long long ncell, const double* params, double* gas, double* aerosol,
+                                    int naer, const int* aer_index, const double* factors, double* gas_wdep,
+                                    double* aer_wdep, double* out, int* stats, double* workspace,
+                                    long long workspace_doubles, void* stream)
 {
+    if (route < CMAQCHEM_KMT2_BY_SIZE || route > CMAQCHEM_KMT2_HAND_OVER) return fail("unknown route");
     if (ncell < 0) return fail("ncell must be >= 0");
     if (ncell == 0) return 0;
     if (!params || !gas || !aerosol || !aer_index || !factors || !gas_wdep || !aer_wdep || !out || !stats ||
@@ -476,8 +488,17 @@ extern "C" int cmaqchem_aqchem_device(long long ncell, const double* params, dou
     a.ncell = ncell;
     a.nlanes = nlanes;
     a.naer = naer;
-    cudaError_t e = launch(k_aqchem_queue, k_aqchem_coop, a, blocks, s);
+    cudaError_t e = launch(k_aqchem_queue, k_aqchem_coop, a, blocks, route, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return fail(std::string("k_aqchem_queue: ") + cudaGetErrorString(e));
     return 0;
+}
+
+extern "C" int cmaqchem_aqchem_device(long long ncell, const double* params, double* gas, double* aerosol, int naer,
+                                      const int* aer_index, const double* factors, double* gas_wdep,
+                                      double* aer_wdep, double* out, int* stats, double* workspace,
+                                      long long workspace_doubles, void* stream)
+{
+    return cmaqchem_diag_aqchem(CMAQCHEM_KMT2_BY_SIZE, ncell, params, gas, aerosol, naer, aer_index, factors, gas_wdep,
+                                aer_wdep, out, stats, workspace, workspace_doubles, stream);
 }

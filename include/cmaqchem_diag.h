@@ -46,6 +46,18 @@ int cmaqchem_diag_step_factor(int device, long long n, const double* maxerr, dou
  * most 96), or -1. */
 int cmaqchem_diag_starved_rows(int device, int feed, int chunks, int* out);
 
+/* cmaqchem_kmt2_solve_device and cmaqchem_aqchem_device (cmaqchem.h) by a route of the caller's: by
+ * the size of the call as they go, every cell in a lane to its end, every cell in a warp (the
+ * cooperative kernels), or in lanes with the last cells handed over to the cooperative kernels.
+ * Same results. */
+enum { CMAQCHEM_KMT2_BY_SIZE = -1, CMAQCHEM_KMT2_LANES = 0, CMAQCHEM_KMT2_COOP = 1, CMAQCHEM_KMT2_HAND_OVER = 2 };
+int cmaqchem_diag_kmt2_solve(int route, long long ncell, const double* params, const double* var_mix,
+                             double* var_out, double* fix_out, int* stats, double* workspace,
+                             long long workspace_doubles, void* stream);
+int cmaqchem_diag_aqchem(int route, long long ncell, const double* params, double* gas, double* aerosol, int naer,
+                         const int* aer_index, const double* factors, double* gas_wdep, double* aer_wdep,
+                         double* out, int* stats, double* workspace, long long workspace_doubles, void* stream);
+
 /* Scheduling knobs of a handle, for the autotuner: "night_pattern" (1: warps whose cells are
  * all dark use the smaller night LU pattern; 0: the day pattern always, same numbers),
  * "lockstep" (work-queue kernel: 0 free-running warps, 1 (default) the block's warps run
