@@ -17,6 +17,10 @@ of a sample of the grid for each candidate:
   and the solves (2), or run free (0, 256-cell blocks only); a lane always refills
   from the queue as soon as its cell finishes.
 
+Calls small enough for the cooperative kernel do not take the work queue; the tuner switches that
+kernel off while it times, so that every candidate is the launch shape it names (the last cells
+are handed over as in larger calls).
+
 Results are cached as JSON keyed by mechanism, GPU name and grid size, so later runs
 on the same machine reuse them.  Every candidate computes bit-identical results (the
 schedule changes no arithmetic), so the choice affects speed only.
@@ -75,14 +79,14 @@ def cache_key(mechanism: str, ncell: int) -> str:
     import torch
     name = torch.cuda.get_device_name() if torch.cuda.is_available() else "cpu"
     bucket = 1 << max(0, int(ncell).bit_length() - 1)     # power-of-two bucket of the grid size
-    return f"{mechanism}|{name}|{bucket}"
+    return f"{mechanism}|{name}|{bucket}|queue"           # what is timed
 
 
 def _time_candidate(g, cand: Candidate, nsteps: int, dev: dict, conc0) -> float:
     s = ChemSolver(g.mech, ncols=g.ncols, nrows=g.nrows, nlays=g.nlays, nspcsd=g.nspcsd,
                    cgrid_index=g.cgrid_index, rtol=1e-3, atol=1e-9, schedule="queue", variant=cand.variant)
     try:
-        s.set_tuning(**cand.knobs())
+        s.set_tuning(ros3_coop=0, **cand.knobs())
         args = [dev[k] for k in KEYS]
         dev["conc"].copy_(conc0)
         s.step(*args)                    # first call from the initial state; gives the queue order
@@ -153,7 +157,7 @@ def sweep(g, specs, ncalls: int = 12, reps: int = 2, verbose: bool = True) -> di
             s = ChemSolver(g.mech, ncols=g.ncols, nrows=g.nrows, nlays=g.nlays, nspcsd=g.nspcsd,
                            cgrid_index=g.cgrid_index, rtol=1e-3, atol=1e-9, schedule="queue", variant=f[0])
             try:
-                s.set_tuning(**knobs)
+                s.set_tuning(ros3_coop=0, **knobs)
                 dev["conc"].copy_(conc0)
                 s.steps(1, *args)
                 dev["conc"].copy_(conc0)
