@@ -99,7 +99,10 @@ def _nvcc() -> str:
 
 
 def sources() -> list[Path]:
-    return sorted(CSRC.glob("*.cu")) + sorted((CSRC / "gen").glob("*.cu"))
+    """The library's translation units: all but SMVGEAR's lane tables, which no kernel reads any more (its
+    programs are in gen/<mech>_coop.cu); the host harness of the Gear tests compiles them."""
+    gen = [p for p in sorted((CSRC / "gen").glob("*.cu")) if not p.name.endswith("_gw_tables.cu")]
+    return sorted(CSRC.glob("*.cu")) + gen
 
 
 def _headers() -> list[Path]:

@@ -97,8 +97,7 @@ def cuda_sources(m: Mechanism, prog: RateProgram, sp: SparseMech, mech: str, src
     units["rates"] = _rconst(m, prog, lay)
     for d in range(2):
         units["rates"] += _feval(m, sp, lay, d) + _explic(m, sp, lay, d)
-    # SMVGEAR uses the day pattern for every cell (see csrc/gear.cuh); the warp-per-cell
-    # kernel runs table-driven cooperative forms of its routines
+    # SMVGEAR uses the day pattern for every cell (see csrc/gear.cuh)
     units["rates"] += _explic(m, sp, lay, 0, gear=True)
     gw_decl, gw_defs, gw_info = _gear_warp_tables(m, sp, lay)
     units["gw_tables"] = gw_defs
@@ -303,9 +302,11 @@ def cuda_sources(m: Mechanism, prog: RateProgram, sp: SparseMech, mech: str, src
 
 
 def _gear_warp_tables(m: Mechanism, sp: SparseMech, lay: Layout) -> tuple[list[str], list[str], dict]:
-    """Tables of the warp-cooperative SMVGEAR routines (day pattern), each listing the
-    operations of the generated sequential routines in an order that lanes can share
-    without changing any element's operation sequence:
+    """Tables of SMVGEAR's routines (day pattern) by lanes.  The kernels run the programs of mechgen/coop.py
+    instead; these tables are kept for the tests that hold them to the sequential routines, and
+    are not part of the library.  Each lists the operations of the generated sequential
+    routines in an order that lanes can share without changing any element's operation
+    sequence:
       rates (RXRAT of each active reaction) and, per species, its derivative terms in
       RBFEVAL's order, species given to lanes longest-first;
       the partial-derivative products (EXPLIC) of 2- and 3-reactant reactions;
