@@ -618,10 +618,13 @@ static int enqueue_step(cmaqchem_handle* h, const chem::GridArgs& a, int itmstep
                     CK(h->ops->ebi_rconst_pass(a, c0, c1, h->d_rki_all, h->d_sun_all, h->nblocks, s));
                 }
                 // A call lasts at least as long as its slowest cell, whose iterations take longer
-                // the more warps share the SM: one per sub-partition up to 256 cells per SM (27,880
-                // CB6r5 cells: 259 ms with 4 warps, 268 with 6, 272 with 8), above that 8 (200,000
-                // cells with 4, 8 and 10: 1,064, 668 and 626 ms; a later call of the hour 212, 149 and
-                // 165 ms).
+                // the more warps share the SM; many cells want more warps.  First and third calls
+                // of CB6r5 with 4 and 8 warps: 252 / 57 and 239 / 60 ms at 130 cells per SM, 301 / 110
+                // and 290 / 113 at 197, 385 / 55 and 302 / 59 at 300, 531 / 111 and 403 / 119 at 510, 751 /
+                // 133 and 533 / 145 at 810 (10 warps 300, 371 and 494 first, 61, 122 and 150 later); of
+                // CRACMM2, which has room for 8: 372 / 121 and 377 / 122 at 25, 417 / 130 and 383 / 134 at
+                // 100, 682 / 167 and 656 / 174 at 200, 672 / 193 and 517 / 197 at 300, 1,000 / 237 and 701 /
+                // 207 at 500.  One per sub-partition, within 9 % either way, up to 256.
                 const long long share = (n + h->nsm - 1) / h->nsm;
                 const int cells = (int)std::min<long long>(share <= 256 ? 4 : std::min(8, h->ops->ebi_max_cells), share);
                 const int nb = (int)std::min<long long>(h->nsm, (n + cells - 1) / cells);
