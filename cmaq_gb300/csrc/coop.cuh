@@ -1,19 +1,20 @@
 // Cooperative ROS3: the lanes of a warp integrate one cell whose state lies in shared memory.
 //
 // The one-cell-per-lane kernels stream a 34 KB workspace per cell from DRAM and need ten
-// thousands of cells to fill the device: a warp's step attempt takes 1.5 ms however few cells
+// thousands of cells to fill the device: a warp's step attempt takes 1.3 ms however few cells
 // there are, because a lone warp issues one FP64 instruction per 64 cycles on GB300.  Here
 // the operations of an attempt (f, the iteration matrix and its factors, the solves) are
 // dealt out to the 32 lanes by a schedule made with the mechanism (mechgen/coop.py: rows of
-// one operation per lane, gen/<mech>_coop.cu), so an attempt of a CB6r5 cell takes 1,440 rows,
-// and the state (25.8 KB, 8 cells per SM; CRACMM2 42.4 KB, 5) stays in shared memory.
+// one operation per lane, gen/<mech>_coop.cu), so an attempt of a CB6r5 cell takes 1,440 rows
+// (19,954 operations in their 46,080 places), and the state (25.8 KB, 8 cells per SM; CRACMM2
+// 42.4 KB, 5) stays in shared memory.
 //
 // Measured (CB6r5): an attempt takes 212,000 cycles for one warp per SM and 285,000 for eight
 // (0.10 and 0.14 ms; the one-cell-per-lane kernel's takes 1.3 ms).  What bounds it: with one
 // warp the latency of a row (126-135 cycles, 64 of them the FP64 instruction's), with eight
 // the FP64 pipe (168 cycles per row of eight warps, 152 at its measured rate).  CHEM calls from
-// the initial state, before and after: 105 cells 124 and 12 ms, 10,527 cells 220 and 61 ms,
-// 36,000 cells 271 and 202 ms; CRACMM2 10,881 cells 701 and 267 ms.
+// the initial state, one cell per lane and here: 105 cells 125 and 11 ms, 11,200 cells 286 and 62 ms,
+// 36,000 cells 392 and 179 ms; CRACMM2 11,200 cells 632 and 250 ms.
 //
 // Every element of a cell's state goes through the same operations in the same order as in
 // the generated sequential routines, and the vector updates below repeat ros3.cuh's, so the

@@ -1,8 +1,8 @@
 // Cooperative EBI: the lanes of a warp integrate one cell whose state lies in shared memory.
 //
 // One Backward-Euler iteration is one pass through the cell's program (coop.cuh: HRRATES,
-// HRG1-HRG4 and HRPRODLOSS dealt out to the lanes by mechgen/coop.py: 192 rows and 16 blocks of
-// divisions, square roots and maxima for CB6r5, 387 and 13 for CRACMM2), then HRSOLVER's species loops over the
+// HRG1-HRG4 and HRPRODLOSS dealt out to the lanes by mechgen/coop.py: 156 rows and 15 blocks of
+// divisions, square roots and maxima for CB6r5, 356 and 15 for CRACMM2), then HRSOLVER's species loops over the
 // lanes with votes for convergence.  Every value is computed with the same operations in the
 // same order as in ebi::iterate and the oracle: same bits.
 //
@@ -10,8 +10,8 @@
 // the latency of an iteration: 26 us, about half of it the rows' (130 cycles each, as in
 // coop.cuh), the rest divisions and the species loops.  The earlier warp kernel walked index
 // tables in global memory and ran the group solutions HRG1-HRG4 on one lane: 0.2 ms.  A first
-// call of 27,880 CB6r5 cells took 881 ms with it and the one-cell-per-lane kernel for the
-// quick cells, and takes 259-272 ms here.
+// call of 27,880 CB6r5 cells took 862-901 ms with it and the one-cell-per-lane kernel for the
+// quick cells, and takes 252-290 ms here (by the inputs).
 #pragma once
 #include "coop.cuh"
 #include "ebi.cuh"

@@ -2,7 +2,7 @@
 // memory.
 //
 // Fun, Jac_SP, KppDecomp and KppSolve are programs of coop.cuh (mechgen/coop.py, from the
-// generated straight-line routines; a step takes 920 rows and 83 blocks of divisions with its
+// generated straight-line routines; a step takes 988 rows and 83 blocks of divisions with its
 // two f, J, factorisation and four solves), the rate laws of Update_RCONST go to a lane each with their
 // temperature factors formed once per cell, and the vectors of Rodas3 are formed over the
 // lanes.  Set-up, mapping and redistribution of a cell (kmt2.cuh with stride 1) run in one
