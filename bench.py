@@ -461,7 +461,7 @@ def run_skewed(device: int, steps: int, tuned) -> dict:
             "step_attempts_per_cell": att}
 
 
-TIGHT_LATEST_S = 1200.0   # the tight leg (about 6 minutes) is skipped when the run has taken longer before it
+TIGHT_LATEST_S = 1200.0   # the tight leg (about 7 minutes) is skipped when the run has taken longer before it
 
 
 def tight_in_time(elapsed_s: float, fn):
@@ -845,7 +845,7 @@ def main():
                     help="only the HETCHEM_RATES kernel on the workload grid's cells, its own JSON line")
     ap.add_argument("--tight-steps", type=int, default=2,
                     help="CHEM calls of the tight-tolerance leg on every 2nd column and 7th layer of the workload "
-                         "grid (0: skip; 2 take about 6 minutes)")
+                         "grid (0: skip; 2 take about 7 minutes)")
     ap.add_argument("--adjoint-dims", default="100x100x35", help="grid of the adjoint window, NCOLSxNROWSxNLAYS")
     ap.add_argument("--only-adjoint", action="store_true",
                     help="time only the adjoint window and print its own line (for profiling)")

@@ -73,13 +73,14 @@ static __device__ __noinline__ bool wait_longer(uint32_t bar, uint32_t t, long l
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(mark) : "r"(bar + 16) : "memory");
     if (__any_sync(0xffffffffu, mark != 0)) return false;
     const auto wait = [&](bool both) {
-        bool there = false;
-        for (const long long t0 = clock64(); !there && __all_sync(0xffffffffu, clock64() - t0 < limit);) {
-            there = try_parity(bar + 8 * (t & 1u), t >> 1 & 1u);
+        // looked for once more after the time is up: a warp that was kept from running has not waited
+        for (const long long t0 = clock64();;) {
+            const bool late = __any_sync(0xffffffffu, clock64() - t0 >= limit);
+            bool there = try_parity(bar + 8 * (t & 1u), t >> 1 & 1u);
             if (both) there = try_parity(bar + 8 * ((t + 1) & 1u), (t + 1) >> 1 & 1u) && there;
             there = __all_sync(0xffffffffu, there);
+            if (there || late) return there;
         }
-        return there;
     };
     if (wait(false)) return true;
     wait(true);
